@@ -54,6 +54,8 @@ struct Handle {
     double* bgd = nullptr;        // 5 x NZ: RHOb, Tb, BXb, BYb, BZb (FP64)
     float* bg32 = nullptr;        // 2 x NZ: RHOb, Tb (FP32)
     PlaneBg* pb = nullptr;        // per interior plane
+    PlaneZ* pz = nullptr;         // per U plane (FP64)
+    MarchRun<double> run{};
     std::vector<double> faz_h, fbz_h, fcz_h;   // host copies of the z stencil factors
     std::vector<double> rka_h, dka_h, ddz_h;   // and of RKAPA, DKAPA, DDZ
     ColC* cxy = nullptr;                       // FP32 column constants: NX in x, then NY in y
@@ -864,6 +866,8 @@ StageArgs make_args(Handle* h)
     a.acc = h->acc;
     a.m = h->m;
     a.s = h->s;
+    a.pz = h->pz;
+    a.run = h->run;
     a.uf = h->uf;
     a.uz = h->uz;
     a.zf = h->zf;
@@ -990,6 +994,7 @@ int destroy(Handle* h)
     cudaFree(h->bgd);
     cudaFree(h->bg32);
     cudaFree(h->pb);
+    cudaFree(h->pz);
     cudaFree(h->cxy);
     cudaFree(h->cbuf);
     cudaFree(h->cbias);
@@ -1267,6 +1272,19 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
         f.ocv = (float)p->ocv; f.omx = (float)p->omx; f.omz = (float)p->omz; f.orm = (float)p->orm;
         f.obeta = (float)p->obeta; f.tmpm = (float)s.tmp_m; f.ogamma = (float)(1.0 / p->gamma);
         f.gamma = (float)p->gamma; f.cw3 = (float)s.cw3;
+    }
+    h->run = MarchRun<double>{p->grav, p->ore, p->c43, p->ore * p->c43, s.tmp_13, s.tmp_a, s.tmp_cond, p->ocv,
+                              p->omx, p->omz, p->orm, p->obeta, s.tmp_m};
+    if (!h->f32) {
+        std::vector<PlaneZ> pz(NZ);
+        for (int u = 0; u < NZ; ++u) {
+            const double az = h->faz_h[u], zp = h->fbz_h[u] + h->fcz_h[u], zm = h->fbz_h[u] - h->fcz_h[u];
+            const double rk = h->rka_h[u], dk = h->dka_h[u];
+            pz[u] = PlaneZ{az, s.tmp_13 * az, p->ore * zp, p->ore * zm, p->orm * zp, p->orm * zm,
+                           rk * zp + dk * az, rk * zm + dk * az, rk, 0.0};
+        }
+        CK(cudaMalloc(&h->pz, sizeof(PlaneZ) * NZ));
+        CK(cudaMemcpy(h->pz, pz.data(), sizeof(PlaneZ) * NZ, cudaMemcpyHostToDevice));
     }
     s.tb = p->tb; s.tp = p->tp; s.tc = p->tc; s.hh = p->hh;
     const double dzs = (double)(1.0f / (float)(npz - 1));

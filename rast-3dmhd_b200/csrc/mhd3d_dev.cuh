@@ -99,6 +99,21 @@ struct Metrics {
     const float *rddx_f, *rddy_f, *rddz_f, *ddx_f, *ddy_f, *ddz_f, *wfz_f;
 };
 
+// per-plane constants of the FP64 column march (march.cuh), one record per U plane
+struct alignas(16) PlaneZ {
+    double az, t13az;      // HZ*DZZDZ, C13*ORE*HZ*DZZDZ
+    double ozp, ozm;       // ORE*(HZ*D2ZZDZ2 +- H2Z*DZZDZ**2)
+    double mzp, mzm;       // ORM times the same
+    double kzp, kzm;       // RKAPA times the same + DKAPA*HZ*DZZDZ
+    double rka, pad;
+};
+
+// run constants of the march (MarchRun in its order)
+template <typename T>
+struct MarchRun {
+    T grav, ore, c43, ore43, t13, tmpa, tmpc, ocv, omx, omz, orm, obeta, tmpm;
+};
+
 struct StageArgs {
     CUtensorMap map_u;      // TMA map of the input U buffer (x, y, z, field)
     CUtensorMap map_z;      // TMA map of Z (x, y, z, field)
@@ -110,6 +125,8 @@ struct StageArgs {
     Accum* acc;
     Metrics m;
     Scalars s;
+    const PlaneZ* pz;       // per U plane (FMA build)
+    MarchRun<double> run;
     size_t uf, uz;          // U: doubles per field, per plane
     size_t zf, zz;          // Z: doubles per field, per plane
     int upitch, zpitch;

@@ -57,6 +57,15 @@ __device__ __forceinline__ void tma_load4(void* dst, const CUtensorMap* map, uns
         : "memory");
 }
 
+// untiled bulk copy of bytes (a multiple of 16, both addresses 16-byte aligned)
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // Periodic halo copies of one interior column: plane offsets of the copies
 // COMMUNICATE makes at I=1/NX and J=1/NY, formed once per thread.
 struct HaloCols {

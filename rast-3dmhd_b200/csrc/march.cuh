@@ -50,9 +50,10 @@ __device__ __forceinline__ float mmul<float>(float a, float b) { return __fmul_r
 template <typename T, bool MAG, bool ROT, bool BG, int BWV, int BS, typename PZ>
 struct March {
     // plane q-1: its cell, read again from its slot (b: without its background)
-    T ru, rv, rw, tt, ro, ri, p, u, v, w;
+    T ru, rv, rw, tt, ro, p, u, v, w;
     T bx, by, bz;
     // carried between arrivals for plane q-1
+    T ri;
     T wx, wy, s;                                 // dw/dx, dw/dy, du/dx + dv/dy
     T fu, fv, fw, fr, ft, heat, w1, w2, w3;      // what its right-hand side holds so far
     T exz, eyz, wz, jx, jy;                      // du/dz + dw/dx, dv/dz + dw/dy, dw/dz, currents: without plane q
@@ -157,11 +158,11 @@ struct March {
     // plane q's x, y terms and its terms from plane q-1 (z: the constants of
     // plane q).  top: it is the top wall, as in complete().
     __device__ __forceinline__ void begin(const T* __restrict__ raw, const T* __restrict__ rip, int o, const PZ& z,
-                                          const T* __restrict__ rawk, const T* __restrict__ ripk, const PZ& zk,
+                                          const T* __restrict__ rawk, const PZ& zk,
                                           const MarchCol<T>& c, const MarchRun<T>& r, bool top, T rwt, T wt, T l1, T l2)
     {
         cell(raw, rip, o, z);
-        recall(rawk, ripk, o, zk);
+        recall(rawk, o, zk);
         if (top) {   // one-sided dRW/dz, dw/dz
             rw = rwt;
             w = wt;
@@ -323,14 +324,13 @@ struct March {
     }
 
     // the cell of plane q-1, from its slot (z: its constants)
-    __device__ __forceinline__ void recall(const T* __restrict__ raw, const T* __restrict__ rip, int o, const PZ& z)
+    __device__ __forceinline__ void recall(const T* __restrict__ raw, int o, const PZ& z)
     {
         ru = ld(raw, F_RU, o);
         rv = ld(raw, F_RV, o);
         rw = ld(raw, F_RW, o);
         tt = ld(raw, F_TT, o);
         ro = ld(raw, F_RO, o);
-        ri = rip[o];
         if (MAG) {
             bx = ld(raw, F_BX, o);
             by = ld(raw, F_BY, o);
@@ -342,9 +342,10 @@ struct March {
         p = pres(ro, tt, z);
     }
 
-    // plane q becomes the carried plane
-    __device__ __forceinline__ void shift()
+    // plane q becomes the carried plane (rq: its 1/RO)
+    __device__ __forceinline__ void shift(T rq)
     {
+        ri = rq;
         wx = nwx;
         wy = nwy;
         s = ns;

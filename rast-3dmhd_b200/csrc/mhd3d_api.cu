@@ -27,10 +27,13 @@ struct Handle {
     int nf = 0;
     int upitch = 0, urows = 0, zpitch = 0, zrows = 0;
     size_t uf = 0, uz = 0, zf = 0, zz = 0;
-    double* ubuf[2] = {nullptr, nullptr};
+    void* ualloc[2] = {nullptr, nullptr};   // the two U allocations
+    double* ubuf[2] = {nullptr, nullptr};   // their column I=1 (floats in the FP32 form)
+    size_t ubytes = 0;
     int cur = 0;               // ubuf[cur] holds the current state
     CUtensorMap map_u[2];      // TMA maps of the two U buffers
     CUtensorMap map_z;
+    CUtensorMap map_o[2];      // tiles without halo of the two U buffers
     CUtensorMap emap_u[2];     // the same for the tile rows of an ensemble (FP32 members)
     CUtensorMap emap_z;
     int ety = 0;               // tile rows emap_* were made for (0: none)
@@ -858,6 +861,7 @@ StageArgs make_args(Handle* h)
     StageArgs a{};
     a.map_u = h->map_u[h->cur];
     a.map_z = h->map_z;
+    a.map_o = h->map_o[h->cur ^ 1];
     a.u_in = h->ubuf[h->cur];
     a.u_out = h->ubuf[h->cur ^ 1];
     a.z = h->z;
@@ -977,8 +981,8 @@ int destroy(Handle* h)
 {
     if (!h) return MHD3D_OK;
     if (h->dev >= 0) cudaSetDevice(h->dev);
-    cudaFree(h->ubuf[0]);
-    cudaFree(h->ubuf[1]);
+    cudaFree(h->ualloc[0]);
+    cudaFree(h->ualloc[1]);
     cudaFree(h->z);
     cudaFree(h->stage);
     cudaFree(h->stage2);
@@ -1026,34 +1030,39 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
     const int NX = npx + 2, NY = npy + 2, NZ = npz + 2;
     h->nf = p->lmag ? 8 : 5;
     h->f32 = p->mode == MHD3D_MODE_FP32;
-    // U: the Fortran index space (halos, ghost planes), rows padded to 16
-    // bytes and to at least one TMA box; Z: interior cells only
-    const int ealign = h->f32 ? 4 : 2;                 // elements per 16 bytes
-    const int bw = h->f32 ? BW32 : BW, bh = h->f32 ? BH32 : BH, ty = h->f32 ? TY32 : TY;
-    h->upitch = (NX + ealign - 1) / ealign * ealign;
-    if (h->upitch < bw) h->upitch = bw;
+    // U: the Fortran index space (halos, ghost planes), rows padded so that the
+    // interior starts a 128-byte line and to at least one TMA box; Z: interior
+    // cells only, rows on 128-byte lines
+    const int line = h->f32 ? 4 : 16;   // FP64: elements of 128 bytes
+    const int uofs = h->f32 ? UOFS32 : UOFS;
+    const int bw = h->f32 ? BX032 + BW32 : BX0 + BW, bh = h->f32 ? BH32 : BH, ty = h->f32 ? TY32 : TY;
+    h->upitch = (std::max(uofs + NX, bw) + line - 1) / line * line;
     h->urows = NY < bh ? bh : NY;
     h->uz = (size_t)h->urows * h->upitch;
     h->uf = (size_t)NZ * h->uz;
-    h->zpitch = (npx + ealign - 1) / ealign * ealign;
+    h->zpitch = (npx + line - 1) / line * line;
     if (h->zpitch < TX) h->zpitch = TX;
     h->zrows = npy < ty ? ty : npy;
     h->zz = (size_t)h->zrows * h->zpitch;
     h->zf = (size_t)npz * h->zz;
     const size_t esize = h->f32 ? sizeof(float) : sizeof(double);
-    const size_t ubytes = esize * h->nf * h->uf;
+    const size_t ubytes = h->ubytes = esize * h->nf * h->uf;
     const size_t zbytes = esize * h->nf * h->zf;
-    CK(cudaMalloc(&h->ubuf[0], ubytes));
-    CK(cudaMalloc(&h->ubuf[1], ubytes));
+    for (int b = 0; b < 2; ++b) {
+        CK(cudaMalloc(&h->ualloc[b], ubytes));
+        CK(cudaMemset(h->ualloc[b], 0, ubytes));
+        h->ubuf[b] = reinterpret_cast<double*>(static_cast<char*>(h->ualloc[b]) + esize * uofs);
+    }
     CK(cudaMalloc(&h->z, zbytes));
-    CK(cudaMemset(h->ubuf[0], 0, ubytes));
-    CK(cudaMemset(h->ubuf[1], 0, ubytes));
     CK(cudaMemset(h->z, 0, zbytes));
     {
         const cuuint64_t du[4] = {(cuuint64_t)h->upitch, (cuuint64_t)h->urows, (cuuint64_t)NZ, (cuuint64_t)h->nf};
-        const cuuint32_t bu[4] = {(cuuint32_t)bw, (cuuint32_t)bh, 1, (cuuint32_t)h->nf};
+        const cuuint32_t bu[4] = {(cuuint32_t)(h->f32 ? BW32 : BW), (cuuint32_t)bh, 1, (cuuint32_t)h->nf};
         for (int b = 0; b < 2; ++b) {
-            int st2 = make_map(&h->map_u[b], h->ubuf[b], du, bu, h->f32);
+            int st2 = make_map(&h->map_u[b], h->ualloc[b], du, bu, h->f32);
+            if (st2) return st2;
+            const cuuint32_t bo[4] = {TX, (cuuint32_t)ty, 1, (cuuint32_t)h->nf};
+            st2 = make_map(&h->map_o[b], h->ualloc[b], du, bo, h->f32);
             if (st2) return st2;
         }
         const cuuint64_t dz[4] = {(cuuint64_t)h->zpitch, (cuuint64_t)h->zrows, (cuuint64_t)npz, (cuuint64_t)h->nf};
@@ -1253,6 +1262,7 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
     s.c13 = p->c13; s.c23 = p->c23; s.c43 = p->c43;
     s.hx = p->hx; s.h2x = p->h2x; s.hy = p->hy; s.h2y = p->h2y; s.hz = p->hz; s.h2z = p->h2z;
     s.gam1 = p->gam1; s.gam2 = p->gam2; s.gam3 = p->gam3; s.zeta1 = p->zeta1; s.zeta2 = p->zeta2;
+    s.zr10 = p->zeta1 / p->gam1;
     s.cv = p->cv; s.ocv = p->ocv; s.ore = p->ore; s.re = p->re; s.repr = p->repr;
     s.theta = p->theta; s.grav = p->grav; s.gamma = p->gamma; s.ogamma = 1.0 / p->gamma; s.sf = p->sf;
     s.rm = p->rm; s.omx = p->omx; s.omz = p->omz; s.orm = p->orm; s.obeta = p->obeta;
@@ -1555,6 +1565,7 @@ int step_async(Handle* h, int n)
             } else {
                 StageArgs a = make_args(h);
                 a.map_u = h->map_u[cur];
+                a.map_o = h->map_o[cur ^ 1];
                 a.u_in = h->ubuf[cur];
                 a.u_out = h->ubuf[cur ^ 1];
                 CK(launch_stage(h, stg, a));
@@ -1868,7 +1879,7 @@ int ens_set_tile(Ensemble* e, int ty)
         const cuuint64_t du[4] = {(cuuint64_t)h->upitch, (cuuint64_t)h->urows, (cuuint64_t)NZ, (cuuint64_t)h->nf};
         const cuuint32_t bu[4] = {(cuuint32_t)BW32, (cuuint32_t)(ty + 2), 1, (cuuint32_t)h->nf};
         for (int b = 0; b < 2; ++b)
-            if (int st = make_map(&h->emap_u[b], h->ubuf[b], du, bu, true)) return st;
+            if (int st = make_map(&h->emap_u[b], h->ualloc[b], du, bu, true)) return st;
         const cuuint64_t dz[4] = {(cuuint64_t)h->zpitch, (cuuint64_t)h->zrows, (cuuint64_t)h->p.npz,
                                   (cuuint64_t)h->nf};
         const cuuint32_t bz[4] = {TX, (cuuint32_t)ty, 1, (cuuint32_t)h->nf};
@@ -2000,11 +2011,11 @@ int ens_tune(Ensemble* e, int steps, int32_t* zlen_out, int32_t* ctas_out, doubl
     std::vector<size_t> ubytes(n);
     for (int i = 0; i < n; ++i) {
         Handle* h = e->mem[i];
-        ubytes[i] = (h->f32 ? sizeof(float) : sizeof(double)) * h->nf * h->uf;
+        ubytes[i] = h->ubytes;
         CK(cudaMalloc(&snap[i], 2 * ubytes[i] + sizeof(Control) + sizeof(Accum)));
         char* b = static_cast<char*>(snap[i]);
-        CK(cudaMemcpyAsync(b, h->ubuf[0], ubytes[i], cudaMemcpyDeviceToDevice, e->st));
-        CK(cudaMemcpyAsync(b + ubytes[i], h->ubuf[1], ubytes[i], cudaMemcpyDeviceToDevice, e->st));
+        CK(cudaMemcpyAsync(b, h->ualloc[0], ubytes[i], cudaMemcpyDeviceToDevice, e->st));
+        CK(cudaMemcpyAsync(b + ubytes[i], h->ualloc[1], ubytes[i], cudaMemcpyDeviceToDevice, e->st));
         CK(cudaMemcpyAsync(b + 2 * ubytes[i], h->ctl, sizeof(Control), cudaMemcpyDeviceToDevice, e->st));
         CK(cudaMemcpyAsync(b + 2 * ubytes[i] + sizeof(Control), h->acc, sizeof(Accum), cudaMemcpyDeviceToDevice,
                            e->st));
@@ -2020,8 +2031,8 @@ int ens_tune(Ensemble* e, int steps, int32_t* zlen_out, int32_t* ctas_out, doubl
         for (int i = 0; i < n; ++i) {
             Handle* h = e->mem[i];
             char* b = static_cast<char*>(snap[i]);
-            CK(cudaMemcpyAsync(h->ubuf[0], b, ubytes[i], cudaMemcpyDeviceToDevice, e->st));
-            CK(cudaMemcpyAsync(h->ubuf[1], b + ubytes[i], ubytes[i], cudaMemcpyDeviceToDevice, e->st));
+            CK(cudaMemcpyAsync(h->ualloc[0], b, ubytes[i], cudaMemcpyDeviceToDevice, e->st));
+            CK(cudaMemcpyAsync(h->ualloc[1], b + ubytes[i], ubytes[i], cudaMemcpyDeviceToDevice, e->st));
             CK(cudaMemcpyAsync(h->ctl, b + 2 * ubytes[i], sizeof(Control), cudaMemcpyDeviceToDevice, e->st));
             CK(cudaMemcpyAsync(h->acc, b + 2 * ubytes[i] + sizeof(Control), sizeof(Accum), cudaMemcpyDeviceToDevice,
                                e->st));

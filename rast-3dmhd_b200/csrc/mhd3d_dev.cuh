@@ -6,10 +6,13 @@
 //              periodic x/y halo at index 0 and NPX+1 / NPY+1, the z ghost
 //              planes at 0 and NPZ+1 (never refreshed by the reference except
 //              RO, which FLUXES inverts there on every call, 3dmhdsub.f:1386-1391
-//              -- the two U buffers carry the two values).  upitch = NPX+2
-//              rounded up to even, so every row starts on 16 bytes and a tile
-//              with its halo is one in-bounds TMA box.  Field-major, x fastest.
-//   Z        : nf fields x NPZ x NPY x zpitch, interior cells only.
+//              -- the two U buffers carry the two values).  Field-major, x
+//              fastest; rows are padded so that the interior starts a 128-byte
+//              line (UOFS).  A pure read-8-write-16-fields march over 512x512x256
+//              doubles measured 2.60 ms with whole lines and 3.58 ms with rows
+//              that start one double into a line.
+//   Z        : nf fields x NPZ x NPY x zpitch, interior cells only, rows on
+//              128-byte lines.
 #pragma once
 
 #ifndef MHD3D_MINB
@@ -28,12 +31,19 @@ namespace mhd3d {
 #define MHD3D_TY 4
 #endif
 #ifndef MHD3D_ZCHUNK
-#define MHD3D_ZCHUNK 64           // planes a CTA marches through (z chunk length target)
+#define MHD3D_ZCHUNK 32           // planes a CTA marches through (z chunk length target)
 #endif
 constexpr int TX = 32;            // tile width (one warp per row)
 constexpr int TY = MHD3D_TY;      // tile rows (threads per CTA = 32*TY)
 constexpr int NT = TX * TY;       // threads per CTA
-constexpr int BW = TX + 2;        // TMA box row: x0-1 .. x0+TX
+// Rows of U start UOFS doubles into their 128-byte aligned storage, so that
+// the interior (I=2, the first cell of tile 0) starts a 128-byte line and a
+// tile's row of a field is two whole lines.  A TMA box starts on 16 bytes:
+// one column before the halo, so a thread's own cell is column tx+BXO of it.
+constexpr int UOFS = 15;          // storage columns before I=1
+constexpr int BXO = 2;
+constexpr int BX0 = UOFS + 1 - BXO;   // storage column of tile 0's box
+constexpr int BW = TX + 4;        // TMA box row: x0-2 .. x0+TX+1
 constexpr int BH = TY + 2;        // TMA box rows: y0-1 .. y0+TY
 constexpr int BSLOT = BW * BH;    // doubles of one field in one plane box
 
@@ -46,6 +56,7 @@ struct Scalars {
     double c13, c23, c43;
     double hx, h2x, hy, h2y, hz, h2z;
     double gam1, gam2, gam3, zeta1, zeta2;
+    double zr10;       // ZETA1/GAM1
     double cv, ocv, ore, re, repr, theta, grav, gamma, ogamma, sf, rm;
     double omx, omz, orm, obeta;
     double tmp_cond;   // OCV/REPR          (3dmhdsub.f:1584)
@@ -117,6 +128,7 @@ struct MarchRun {
 struct StageArgs {
     CUtensorMap map_u;      // TMA map of the input U buffer (x, y, z, field)
     CUtensorMap map_z;      // TMA map of Z (x, y, z, field)
+    CUtensorMap map_o;      // tiles without halo of the output U buffer (stage 2 of the FMA build)
     const double* u_in;     // current state
     double* u_out;          // next state (other ping-pong buffer)
     double* z;              // Z (read in stages 2,3; written in stages 1,2)
@@ -152,6 +164,9 @@ struct StageArgs {
 #endif
 constexpr int TY32 = MHD3D_TY32;        // tile rows of the FP32 kernel
 constexpr int NT32 = TX * TY32;
+constexpr int UOFS32 = 0;               // storage columns before I=1
+constexpr int BXO32 = 1;                // own cell in a box row
+constexpr int BX032 = 0;
 constexpr int BW32 = 36;                // TMA box row: x0-1 .. x0+34 (36 floats = 144 B, a 16-B multiple)
 constexpr int BH32 = TY32 + 2;
 constexpr int BSLOT32 = BW32 * BH32;
@@ -231,20 +246,17 @@ __host__ __device__ inline double of_key(unsigned long long k)
 // Launchers, one set per arithmetic mode (compiled from the same source
 // with and without FMA contraction).
 namespace exact {
-size_t stage_smem_bytes(int lmag);
 cudaError_t launch_stage(int stage, const StageArgs& a, cudaStream_t st);
 cudaError_t launch_cfl(const StageArgs& a, cudaStream_t st);
 cudaError_t launch_bcon(const StageArgs& a, cudaStream_t st);
 }
 namespace fast {
-size_t stage_smem_bytes(int lmag);
 cudaError_t launch_stage(int stage, const StageArgs& a, cudaStream_t st);
 cudaError_t launch_cfl(const StageArgs& a, cudaStream_t st);
 cudaError_t launch_bcon(const StageArgs& a, cudaStream_t st);
 }
 // FP32 form (FMA contraction, FP64 CFL reduction)
 namespace f32 {
-size_t stage_smem_bytes(int lmag);
 cudaError_t launch_stage(int stage, const StageArgs32& a, cudaStream_t st);
 cudaError_t launch_cfl(const StageArgs32& a, cudaStream_t st);
 // persistent multi-grid form (ensembles) with tile rows ty (2, 4 or 8): args,

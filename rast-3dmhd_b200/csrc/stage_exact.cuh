@@ -8,24 +8,32 @@ enum Q { Q_RU = 0, Q_RV, Q_RW, Q_RO, Q_TT, Q_RI, Q_UU, Q_VV, Q_WW, Q_P, Q_BX, Q_
 // Of the ring's slots planes k-1, k, k+1 are in use and plane k+2 is in flight.
 constexpr int NRI = 3;    // 1/RO ring slots (planes k-1, k, k+1)
 
-template <bool MAG>
+constexpr int RIW = TX + 2;          // 1/RO rows: x0-1 .. x0+TX
+constexpr int RIS = RIW * BH;
+
+// Three CTAs an SM leave 76,800 bytes a CTA: the mbarriers and the flag sit in
+// the gap before the Z slots, and the base needs no alignment slack.
+template <bool MAG, int STAGE = 0>
 struct Lay {
     static constexpr int NF = MAG ? 8 : 5;
     static constexpr int RAW_SLOT = (NF * BSLOT * 8 + 127) / 128 * 128 / 8;   // doubles, 128-B aligned
     static constexpr int ZT = NF * TY * TX;                                   // Z tile doubles
     static constexpr int RI_OFF = NRAW * RAW_SLOT;
-    static constexpr int Z_OFF = ((RI_OFF + NRI * BSLOT) * 8 + 127) / 128 * 128 / 8;
-    static constexpr int BAR_OFF = Z_OFF + 2 * ZT;       // two Z slots; NRAW+2 <= 8 mbarriers (8 B each)
-    static constexpr int RED_OFF = BAR_OFF + 8;          // CFL block reduction
-    static constexpr int FLAG_OFF = RED_OFF + (NT / 32) * 8;   // three keys per warp
-    static constexpr int TOTAL = FLAG_OFF + 2;
-    static constexpr size_t BYTES = (size_t)TOTAL * 8 + 128;   // + alignment slack
+    static constexpr int BAR_OFF = RI_OFF + NRI * RIS;   // NRAW+2 mbarriers (8 B each), then the flag
+    static constexpr int FLAG_OFF = BAR_OFF + NRAW + 2;
+    static constexpr int Z_OFF = ((FLAG_OFF + 1) * 8 + 127) / 128 * 128 / 8;
+    static constexpr int RED_OFF = Z_OFF + 2 * ZT;       // two Z slots, then the CFL block reduction:
+    static constexpr int TOTAL = RED_OFF + (NT / 32) * 3;   // three keys per warp
+    static constexpr size_t BYTES = (size_t)TOTAL * 8;
 };
+#if MHD3D_MINB == 3
+static_assert(Lay<true>::BYTES <= 76800, "three CTAs an SM");
+#endif
 
 // value of quantity QQ at offset off of a plane slot: raw fields, 1/RO, and the
 // products FLUXES forms on the whole array (UU=RU*RO' with RO'=1/RO, WW1=RO*TT)
 template <int QQ>
-__device__ __forceinline__ double qv(const double* __restrict__ raw, const double* __restrict__ ri, int off)
+__device__ __forceinline__ double qv(const double* __restrict__ raw, const double* __restrict__ ri, int off, int ro)
 {
     if constexpr (QQ == Q_RU) return raw[F_RU * BSLOT + off];
     else if constexpr (QQ == Q_RV) return raw[F_RV * BSLOT + off];
@@ -35,10 +43,10 @@ __device__ __forceinline__ double qv(const double* __restrict__ raw, const doubl
     else if constexpr (QQ == Q_BX) return raw[F_BX * BSLOT + off];
     else if constexpr (QQ == Q_BY) return raw[F_BY * BSLOT + off];
     else if constexpr (QQ == Q_BZ) return raw[F_BZ * BSLOT + off];
-    else if constexpr (QQ == Q_RI) return ri[off];
-    else if constexpr (QQ == Q_UU) return raw[F_RU * BSLOT + off] * ri[off];
-    else if constexpr (QQ == Q_VV) return raw[F_RV * BSLOT + off] * ri[off];
-    else if constexpr (QQ == Q_WW) return raw[F_RW * BSLOT + off] * ri[off];
+    else if constexpr (QQ == Q_RI) return ri[ro];
+    else if constexpr (QQ == Q_UU) return raw[F_RU * BSLOT + off] * ri[ro];
+    else if constexpr (QQ == Q_VV) return raw[F_RV * BSLOT + off] * ri[ro];
+    else if constexpr (QQ == Q_WW) return raw[F_RW * BSLOT + off] * ri[ro];
     else return raw[F_RO * BSLOT + off] * raw[F_TT * BSLOT + off];
 }
 
@@ -49,12 +57,10 @@ __device__ __forceinline__ double qv(const double* __restrict__ raw, const doubl
 template <bool MAG, bool ROT, int STAGE>
 __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant__ StageArgs a)
 {
-    using L = Lay<MAG>;
+    using L = Lay<MAG, STAGE>;
     constexpr int NF = L::NF;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    // 128-byte aligned base, formed by pointer arithmetic on the shared array
-    // so that every access below stays a shared-window (32-bit) access
-    double* const sbase = reinterpret_cast<double*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
+    double* const sbase = reinterpret_cast<double*>(smem_raw);
     double* const sraw = sbase;
     double* const sri = sbase + L::RI_OFF;
     double* const sz = sbase + L::Z_OFF;
@@ -76,7 +82,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     const int k1 = (chunk == a.nchunks - 1) ? npz : k0 + a.zlen;
     const int gi = x0 + tx, gj = y0 + ty;
     const bool active = gi < npx && gj < npy;
-    const int lx = tx + 1, ly = ty + 1;
+    const int lx = tx + BXO, ly = ty + 1;
 
     const double DT = ctl->dt;
     const double cu = STAGE == 1 ? s.gam1 * DT : STAGE == 2 ? s.gam2 * DT : s.gam3 * DT;   // COEF for U
@@ -121,14 +127,18 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
         const int sl = (kp + 1) % NRAW;
         fence_proxy_async();
         mbar_expect_tx(&bars[sl], raw_bytes);
-        tma_load4(sraw + (size_t)sl * L::RAW_SLOT, &a.map_u, &bars[sl], x0, y0, kp + 1, 0);
+        tma_load4(sraw + (size_t)sl * L::RAW_SLOT, &a.map_u, &bars[sl], x0 + BX0, y0, kp + 1, 0);
         hi_issued = kp;
     };
     auto parity_of = [&](int kp) -> unsigned { return (unsigned)(((kp - (k0 - 1)) / NRAW) & 1); };
     auto derive_ri = [&](int kp) {
         const double* r = sraw + (size_t)((kp + 1) % NRAW) * L::RAW_SLOT + F_RO * BSLOT;
-        double* d = sri + (size_t)((kp + 1) % 3) * BSLOT;
-        for (int p = tid; p < BSLOT; p += NT) d[p] = 1.0 / r[p];
+        double* d = sri + (size_t)((kp + 1) % 3) * RIS;
+        // a warp a row, then the last BH-TY rows and the two columns beyond a warp
+        auto put = [&](int y, int x) { d[y * RIW + x] = 1.0 / r[y * BW + x + BXO - 1]; };
+        put(ty, tx);
+        if (ty < BH - TY) put(TY + ty, tx);
+        else if (ty == BH - TY && tx < 2 * BH) put(tx >> 1, TX + (tx & 1));
     };
 
     // Z of plane kp (stages 2, 3) goes to slot (kp-k0)&1, a plane ahead of its
@@ -174,12 +184,12 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
             const double* Rm = sraw + (size_t)((k + 0) % NRAW) * L::RAW_SLOT;   // plane k-1
             const double* Rc = sraw + (size_t)((k + 1) % NRAW) * L::RAW_SLOT;   // plane k
             const double* Rp = sraw + (size_t)((k + 2) % NRAW) * L::RAW_SLOT;   // plane k+1
-            const double* Im = sri + (size_t)((k + 0) % 3) * BSLOT;
-            const double* Ic = sri + (size_t)((k + 1) % 3) * BSLOT;
-            const double* Ip = sri + (size_t)((k + 2) % 3) * BSLOT;
-#define C_(q, dx, dy) qv<q>(Rc, Ic, (ly + (dy)) * BW + (lx + (dx)))
-#define M_(q, dx, dy) qv<q>(Rm, Im, (ly + (dy)) * BW + (lx + (dx)))
-#define P_(q, dx, dy) qv<q>(Rp, Ip, (ly + (dy)) * BW + (lx + (dx)))
+            const double* Im = sri + (size_t)((k + 0) % 3) * RIS;
+            const double* Ic = sri + (size_t)((k + 1) % 3) * RIS;
+            const double* Ip = sri + (size_t)((k + 2) % 3) * RIS;
+#define C_(q, dx, dy) qv<q>(Rc, Ic, (ly + (dy)) * BW + (lx + (dx)), (ly + (dy)) * RIW + (tx + 1 + (dx)))
+#define M_(q, dx, dy) qv<q>(Rm, Im, (ly + (dy)) * BW + (lx + (dx)), (ly + (dy)) * RIW + (tx + 1 + (dx)))
+#define P_(q, dx, dy) qv<q>(Rp, Ip, (ly + (dy)) * BW + (lx + (dx)), (ly + (dy)) * RIW + (tx + 1 + (dx)))
 #define WALL_LOADS                                                                                   \
     double rw2 = 0, ww2 = 0, bx2 = 0, bx3 = 0, by2 = 0, by3 = 0;                                     \
     if (top || bot) {                                                                                \

@@ -15,7 +15,7 @@
 //
 // Work decomposition and plane ring as in the FP64 kernel: a CTA owns a
 // 32 x TY32 tile of columns and a chunk of z planes; planes arrive by TMA
-// (box 36 x (TY32+2) x 1 x nf floats) into a four-slot ring, Z by its own box;
+// (box BW32 x (TY32+2) x 1 x nf floats) into a four-slot ring, Z by its own box;
 // every wait is bounded.  No TMA load uses cluster multicast.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -174,7 +174,7 @@ __device__ __forceinline__ void stage32_item(const StageArgs32& a, const int til
     const int k1 = (chunk == a.nchunks - 1) ? npz : k0 + a.zlen;
     const int gi = x0 + tx, gj = y0 + ty;
     const bool active = gi < npx && gj < npy;
-    const int lx = tx + 1, ly = ty + 1;
+    const int lx = tx + BXO32, ly = ty + 1;
 
     const double DT = ctl->dt;
     const float cu = (float)(STAGE == 1 ? s.gam1 * DT : STAGE == 2 ? s.gam2 * DT : s.gam3 * DT);
@@ -219,8 +219,8 @@ __device__ __forceinline__ void stage32_item(const StageArgs32& a, const int til
         const int sl = (kp + 1) & 3;
         fence_proxy_async();
         mbar_expect_tx(&bars[sl], raw_bytes);
-        tma_load4(reinterpret_cast<unsigned char*>(sraw) + (size_t)sl * L::RAW_SLOT_B, &a.map_u, &bars[sl], x0, y0,
-                  kp + 1, 0);
+        tma_load4(reinterpret_cast<unsigned char*>(sraw) + (size_t)sl * L::RAW_SLOT_B, &a.map_u, &bars[sl], x0 + BX032,
+                  y0, kp + 1, 0);
         hi_issued = kp;
     };
     auto parity_of = [&](int kp) -> unsigned { return (unsigned)(((kp - (k0 - 1)) >> 2) & 1); };
@@ -738,8 +738,6 @@ cudaError_t launch_stage(int stage, const StageArgs32& a, cudaStream_t st)
     if (a.s.lmag) return a.s.lrot ? launch_stage_t<true, true>(stage, a, st) : launch_stage_t<true, false>(stage, a, st);
     return a.s.lrot ? launch_stage_t<false, true>(stage, a, st) : launch_stage_t<false, false>(stage, a, st);
 }
-
-size_t stage_smem_bytes(int lmag) { return lmag ? Lay32<true>::BYTES : Lay32<false>::BYTES; }
 
 template <bool MAG, bool ROT, int TYV>
 static cudaError_t launch_multi_t(int stage, const StageArgs32* args, const int* order, const int* item_base,

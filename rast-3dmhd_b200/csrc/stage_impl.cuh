@@ -189,12 +189,12 @@ __global__ void __launch_bounds__(NT) k_bcon(const __grid_constant__ StageArgs a
 template <bool MAG, bool ROT>
 static cudaError_t launch_stage_t(int stage, const StageArgs& a, cudaStream_t st)
 {
-    const size_t smem = Lay<MAG>::BYTES;
     const int nty = (a.s.npy + TY - 1) / TY;
     dim3 grid(a.ntx * nty, a.nchunks);
     switch (stage) {
 #define L_(S)                                                                                              \
     case S: {                                                                                              \
+        constexpr size_t smem = Lay<MAG, S>::BYTES;                                                        \
         static std::atomic<unsigned long long> attr_set{0};                                                \
         cudaError_t ae = smem_attr_once(attr_set, reinterpret_cast<const void*>(k_stage<MAG, ROT, S>), smem); \
         if (ae != cudaSuccess) return ae;                                                                  \
@@ -214,8 +214,6 @@ cudaError_t launch_stage(int stage, const StageArgs& a, cudaStream_t st)
     if (a.s.lmag) return a.s.lrot ? launch_stage_t<true, true>(stage, a, st) : launch_stage_t<true, false>(stage, a, st);
     return a.s.lrot ? launch_stage_t<false, true>(stage, a, st) : launch_stage_t<false, false>(stage, a, st);
 }
-
-size_t stage_smem_bytes(int lmag) { return lmag ? Lay<true>::BYTES : Lay<false>::BYTES; }
 
 cudaError_t launch_cfl(const StageArgs& a, cudaStream_t st)
 {

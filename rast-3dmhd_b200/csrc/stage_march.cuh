@@ -1,16 +1,25 @@
 // stage_march.cuh -- the stage kernel of the FMA build, included by
 // stage_impl.cuh: the column march of march.cuh in FP64.
 //
-// Bound by the latency of its instructions at 12 warps an SM (a plane holds
-// 705 instructions a thread in stage 1, 321 of them FP64) and, at the largest
-// grids, by DRAM.  Reading each plane as it arrives instead of planes k-1, k,
-// k+1 for every cell leaves two planes in flight instead of one and took a
-// step at 256x256x128 from 1583 to 1400 us, at 512x512x256 from 10.2 to
-// 9.95 ms and of a 203x150x75 run without magnetic field from 376 to 350 us.
-// Tried against this form in the same run: 4 CTAs an SM at 128 registers with
-// a three-slot ring and one Z slot 1425 us and 10.4 ms; 32x8 tiles, 2 CTAs an
+// Stage 1 writes no Z: Z = U1 + ZETA1*DT*F1 follows in stage 2 from U1 and the
+// state U0 the step began with, which is still in the buffer stage 2 writes
+// (a cell is read by the thread that then overwrites it, and by no other).
+// That is 64 of the 640 bytes a cell and step, and one rounding less: errors
+// against 80-bit arithmetic fall by 13-15 % in every field.
+//
+// Bound by DRAM traffic in flight (12 warps an SM, two planes in the ring
+// beyond the two in use, three in stage 1) together with the latency of a
+// plane's 705-830 instructions.  Measured at 512x512x256 (ms a step; stages):
+// one plane in flight, planes k-1, k, k+1 read for every cell 10.61 (3.18 /
+// 3.58 / 3.79); the march 9.76 (2.98 / 3.31 / 3.37); stage 1 without Z, rows
+// on 128-byte lines and 32-plane chunks 9.39 (2.62 / 3.24 / 3.39).  At
+// 256x256x128 1581, 1413 and 1241 us.
+// Tried against the march in one run: 4 CTAs an SM at 128 registers with a
+// three-slot ring and one Z slot 1425 us and 10.4 ms; 32x8 tiles, 2 CTAs an
 // SM, three slots 1410 us and 10.16 ms, four slots and one Z slot 1529 us and
-// 10.8 ms.
+// 10.8 ms; planes 1, 2, 4 beyond the ring prefetched into L2 10.09, 10.52,
+// 11.64 ms against 9.91 (neighbours' halo rows leave L2 earlier).
+
 // 1/x by two Newton-Raphson steps y <- y + y(1 - xy) from the approximate
 // reciprocal rcp.approx.ftz.f64 (each step squares the relative error, so
 // two reach the rounding level): within an ulp or so of the correctly rounded
@@ -26,16 +35,17 @@ __device__ __forceinline__ double recip(double x)
     return fma(y, e, y);
 }
 
-constexpr int NZS = 2;   // Z slots
-template <bool MAG>
+constexpr int NZS = 2;   // Z slots (stages 2, 3)
+template <bool MAG, int STAGE>
 struct Lay {
     static constexpr int NF = MAG ? 8 : 5;
+    static constexpr int NR = STAGE >= 2 ? NRAW : NRAW + 1;   // ring slots: stages without Z hold a plane more
     static constexpr int REC = (NF * BSLOT * 8 + 127) / 128 * 128 / 8;   // plane constants behind the fields
     static constexpr int RAW_SLOT = REC + 16;
     static constexpr int ZT = NF * TY * TX;
-    static constexpr int RI_OFF = NRAW * RAW_SLOT;
-    static constexpr int Z_OFF = ((RI_OFF + 3 * BSLOT) * 8 + 127) / 128 * 128 / 8;
-    static constexpr int BAR_OFF = Z_OFF + NZS * ZT;
+    static constexpr int RI_OFF = NR * RAW_SLOT;
+    static constexpr int Z_OFF = ((RI_OFF + 2 * BSLOT) * 8 + 127) / 128 * 128 / 8;
+    static constexpr int BAR_OFF = Z_OFF + (STAGE >= 2 ? NZS : 0) * ZT;
     static constexpr int RED_OFF = BAR_OFF + 8;
     static constexpr int FLAG_OFF = RED_OFF + (NT / 32) * 8;
     static constexpr int TOTAL = FLAG_OFF + 2;
@@ -47,7 +57,8 @@ struct Lay {
 template <bool MAG, bool ROT, int STAGE>
 __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant__ StageArgs a)
 {
-    using L = Lay<MAG>;
+    using L = Lay<MAG, STAGE>;
+    constexpr int NR = L::NR;
     using Mc = March<double, MAG, ROT, false, BW, BSLOT, PlaneZ>;
     constexpr int NF = L::NF;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -74,11 +85,11 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     const int k1 = (chunk == a.nchunks - 1) ? npz : k0 + a.zlen;
     const int gi = x0 + tx, gj = y0 + ty;
     const bool active = gi < npx && gj < npy;
-    const int o = (ty + 1) * BW + tx + 1;   // own cell in a plane slot
+    const int o = (ty + 1) * BW + tx + BXO;   // own cell in a plane slot
 
     const double DT = ctl->dt;
     const double cu = STAGE == 1 ? s.gam1 * DT : STAGE == 2 ? s.gam2 * DT : s.gam3 * DT;
-    const double cz = STAGE == 1 ? s.zeta1 * DT : s.zeta2 * DT;
+    const double cz = s.zeta2 * DT;
     const double C13 = s.c13, C23 = s.c23, C43 = s.c43;
     MarchCol<double> col;
     {
@@ -101,7 +112,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
         const bool stopped = STAGE != 0 && ctl->stop;
         *sflag = stopped ? -1 : 0;
         if (!stopped) {
-            for (int i = 0; i < NRAW + NZS; ++i) mbar_init(&bars[i], 1);
+            for (int i = 0; i < NR + NZS; ++i) mbar_init(&bars[i], 1);
             fence_mbar_init();
         }
     }
@@ -115,40 +126,42 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     __syncthreads();
     if (*sflag < 0) return;
 
-    // plane q (-1 .. npz) is fill n = q-(k0-1) of the CTA: raw slot n % NRAW,
-    // 1/RO slot n % 3; the plane's constants arrive with it
+    // plane q (-1 .. npz) is fill n = q-(k0-1) of the CTA: raw slot n % NR,
+    // 1/RO slot n & 1; the plane's constants arrive with it
     int hi_issued = k0 - 2;
     auto issue_plane = [&](int q) {
-        const int sl = (q - (k0 - 1)) % NRAW;
+        const int sl = (q - (k0 - 1)) % NR;
         fence_proxy_async();
         mbar_expect_tx(&bars[sl], raw_bytes);
-        tma_load4(sbase + (size_t)sl * L::RAW_SLOT, &a.map_u, &bars[sl], x0, y0, q + 1, 0);
+        tma_load4(sbase + (size_t)sl * L::RAW_SLOT, &a.map_u, &bars[sl], x0 + BX0, y0, q + 1, 0);
         bulk_load(sbase + (size_t)sl * L::RAW_SLOT + L::REC, a.pz + (q + 1), (unsigned)sizeof(PlaneZ), &bars[sl]);
         hi_issued = q;
     };
     auto wait_plane = [&](int q, long limit) -> bool {
         const int n = q - (k0 - 1);
-        return mbar_wait(&bars[n % NRAW], (unsigned)(n / NRAW) & 1u, limit);
+        return mbar_wait(&bars[n % NR], (unsigned)(n / NR) & 1u, limit);
     };
     auto derive_ri = [&](int q) {
         const int n = q - (k0 - 1);
-        const double* r = sbase + (size_t)(n % NRAW) * L::RAW_SLOT + F_RO * BSLOT;
-        double* d = sri + (size_t)(n % 3) * BSLOT;
+        const double* r = sbase + (size_t)(n % NR) * L::RAW_SLOT + F_RO * BSLOT;
+        double* d = sri + (size_t)(n & 1) * BSLOT;
         for (int p = tid; p < BSLOT; p += NT) d[p] = recip(r[p]);
     };
     int z_hi = k0 - 1;
     auto issue_z = [&](int k) {
         const int zs = (k - k0) % NZS;
         fence_proxy_async();
-        mbar_expect_tx(&bars[NRAW + zs], z_bytes);
-        tma_load4(sz + (size_t)zs * L::ZT, &a.map_z, &bars[NRAW + zs], x0, y0, k, 0);
+        mbar_expect_tx(&bars[NR + zs], z_bytes);
+        // stage 2: the state the step began with, still in the output buffer
+        if (STAGE == 2) tma_load4(sz + (size_t)zs * L::ZT, &a.map_o, &bars[NR + zs], x0 + UOFS + 1, y0 + 1, k + 1, 0);
+        else tma_load4(sz + (size_t)zs * L::ZT, &a.map_z, &bars[NR + zs], x0, y0, k, 0);
         z_hi = k;
     };
     auto wait_z = [&](int k) -> bool {
-        return mbar_wait(&bars[NRAW + (k - k0) % NZS], (unsigned)(((k - k0) / NZS) & 1));
+        return mbar_wait(&bars[NR + (k - k0) % NZS], (unsigned)(((k - k0) / NZS) & 1));
     };
     if (tid == 0) {
-        for (int q = k0 - 1; q <= k0 - 2 + NRAW && q <= k1; ++q) issue_plane(q);
+        for (int q = k0 - 1; q <= k0 - 2 + NR && q <= k1; ++q) issue_plane(q);
         if (STAGE >= 2) {
             for (int k = k0; k < k0 + NZS && k < k1; ++k) issue_z(k);
         }
@@ -162,13 +175,12 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     Mc c;
     bool zok = true;
     if (!*sflag) {
-        int slot = 0, pslot = NRAW - 1, rslot = 0, prslot = 2;   // of planes q and q-1
+        int slot = 0, pslot = NR - 1;   // of planes q and q-1
 #pragma unroll 1
         for (int q = k0 - 1; q <= k1; ++q) {
             const double* const raw = sbase + (size_t)slot * L::RAW_SLOT;
-            const double* const rip = sri + (size_t)rslot * BSLOT;
+            const double* const rip = sri + (size_t)((q - (k0 - 1)) & 1) * BSLOT;
             const double* const rawk = sbase + (size_t)pslot * L::RAW_SLOT;
-            const double* const ripk = sri + (size_t)prslot * BSLOT;
             const int k = q - 1;   // the plane this arrival completes
             if (active) {
                 const PlaneZ& zq = *reinterpret_cast<const PlaneZ*>(raw + L::REC);
@@ -176,7 +188,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                 c.arrive(raw, rip, o, col);
                 if (q > k0) {
                     c.cell(raw, rip, o, zq);
-                    c.recall(rawk, ripk, o, zk);
+                    c.recall(rawk, o, zk);
                     const bool top = (k == 0), bot = (k == npz - 1), wall = top || bot;
                     const double ghost = c.nri;
                     double l1 = 0.0, l2 = 0.0;
@@ -227,6 +239,19 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                                 zby = zt_[F_BY * NT];
                                 zbz = zt_[F_BZ * NT];
                             }
+                            if (STAGE == 2) {
+                                // Z = U1 + ZETA1*DT*F1 with GAM1*DT*F1 = U1 - U0
+                                zu = fma(s.zr10, c.ru - zu, c.ru);
+                                zv = fma(s.zr10, c.rv - zv, c.rv);
+                                zw = fma(s.zr10, c.rw - zw, c.rw);
+                                zt = fma(s.zr10, c.tt - zt, c.tt);
+                                zr = fma(s.zr10, c.ro - zr, c.ro);
+                                if (MAG) {
+                                    zbx = fma(s.zr10, c.bx - zbx, c.bx);
+                                    zby = fma(s.zr10, c.by - zby, c.by);
+                                    zbz = fma(s.zr10, c.bz - zbz, c.bz);
+                                }
+                            }
                         }
                         const double nu = zu + cu * c.fu, nv = zv + cu * c.fv, nw = zw + cu * c.fw;
                         const double nr = zr + cu * c.fr, nt = zt + cu * c.ft;
@@ -240,9 +265,9 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                                               {nr, nbx, nby, nu, nv, nw, nt, nbz});
                             else
                                 store_cell<5>(pl, a.uf, ucol, hc, {F_RO, F_RU, F_RV, F_RW, F_TT}, {nr, nu, nv, nw, nt});
-                            // Z for the next stage: Z = U + ZETA*DT*F; on the
-                            // walls only RO, BX, BY are ever read back
-                            if (STAGE < 3) {
+                            // Z for stage 3: Z = U + ZETA*DT*F; on the walls only
+                            // RO, BX, BY are ever read back
+                            if (STAGE == 2) {
                                 double* zo = a.z + zc;
                                 zo[F_RO * a.zf] = nr + cz * c.fr;
                                 if (MAG) {
@@ -325,7 +350,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                     asm volatile("" ::: "memory");
                     if (top) {
                         // ghost RO plane: FLUXES leaves 1/RO behind (3dmhdsub.f:1386-1391)
-                        if (STAGE != 0) store_cell<1>(a.u_out, a.uf, ucol, hc, {F_RO}, {ripk[o]});
+                        if (STAGE != 0) store_cell<1>(a.u_out, a.uf, ucol, hc, {F_RO}, {c.ri});
                         const double* u = a.u_in + ucol + 2 * a.uz;
                         const double* u2 = u + a.uz;
                         const double rwp = u[F_RW * a.uf], rw2 = u2[F_RW * a.uf];
@@ -337,9 +362,9 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                             l2 = Mc::wall_d2(zq, 1.0, raw[F_BY * BSLOT + o], u[F_BY * a.uf], u2[F_BY * a.uf], u3[F_BY * a.uf]);
                         }
                     }
-                    c.begin(raw, rip, o, zq, rawk, ripk, zk, col, run, top, rwt, wt, l1, l2);
+                    c.begin(raw, rip, o, zq, rawk, zk, col, run, top, rwt, wt, l1, l2);
                 }
-                c.shift();
+                c.shift(rip[o]);
             } else if (STAGE >= 2 && q > k0) {
                 // columns outside the domain still see the Z fill of this plane land
                 zok = wait_z(k);
@@ -354,20 +379,18 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
             if (*sflag) break;
             // the slot of plane q-1 and, from q = k0+1 on, the Z slot of plane q-1 are free
             if (tid == 0) {
-                if (q >= k0 && q - 1 + NRAW <= k1) issue_plane(q - 1 + NRAW);
+                if (q >= k0 && q - 1 + NR <= k1) issue_plane(q - 1 + NR);
                 if (STAGE >= 2 && q > k0 && q - 1 + NZS < k1) issue_z(q - 1 + NZS);
             }
             pslot = slot;
-            slot = slot + 1 == NRAW ? 0 : slot + 1;
-            prslot = rslot;
-            rslot = rslot == 2 ? 0 : rslot + 1;
+            slot = slot + 1 == NR ? 0 : slot + 1;
         }
     }
     if (*sflag) {
         // a bounded wait gave up: let every fill still in flight land (again
         // bounded), report, and leave without touching the reduction
         if (tid == 0) {
-            for (int q = hi_issued - (NRAW - 1); q <= hi_issued; ++q)
+            for (int q = hi_issued - (NR - 1); q <= hi_issued; ++q)
                 if (q >= k0 - 1) wait_plane(q, WAIT_LIMIT);
             for (int k = z_hi - (NZS - 1); k <= z_hi; ++k)
                 if (k >= k0) wait_z(k);

@@ -49,7 +49,7 @@ struct Handle {
     Accum* acc = nullptr;
     Metrics m{};
     Scalars s{};
-    int ntx = 0, zlen = 0, nchunks = 0;
+    int ntx = 0, nchunks = 0;
     bool dt_valid = false;
     unsigned long long w4key = ~0ull;   // key of min over cells of W4 (MHD), else ~0
     // FP32 form: the buffers above hold floats; background profiles
@@ -879,7 +879,6 @@ StageArgs make_args(Handle* h)
     a.upitch = h->upitch;
     a.zpitch = h->zpitch;
     a.ntx = h->ntx;
-    a.zlen = h->zlen;
     a.nchunks = h->nchunks;
     a.wait_first = h->wait_first;
     return a;
@@ -921,7 +920,6 @@ StageArgs32 make_args32(Handle* h)
     a.upitch = h->upitch;
     a.zpitch = h->zpitch;
     a.ntx = h->ntx;
-    a.zlen = h->zlen;
     a.nchunks = h->nchunks;
     return a;
 }
@@ -1009,6 +1007,37 @@ int destroy(Handle* h)
     if (h->own) cudaStreamDestroy(h->own);
     delete h;
     return MHD3D_OK;
+}
+
+// Number of z chunks of a grid of `tiles` tile columns when `slots` CTAs are
+// resident at once: the least of waves x (planes a chunk + 0.7), where the
+// last, partly filled wave counts as a whole one up to four waves (all CTAs
+// of a wave end together) and as half a wave on average beyond; chunks of at
+// most 40 planes, so that neighbouring tiles stay close enough in z to find
+// each other's halo rows in L2, and of at least three (BCON reads the two
+// planes next to a wall from the wall's own chunk).  The 0.7 is the fill of
+// the ring as the sweeps below see it.  Against the best of a sweep over the
+// number of chunks (1 to 64; FP64, reference rounding and FP32, 64x64x48 to
+// 512x512x256, ragged ones among them) the rule's choice takes 1.00 to 1.05
+// times as long.  A fixed 32-plane target that also aimed at two waves, with
+// the remainder left to the last chunk, took 1.58 times (96x96x64 in reference
+// rounding, 278 us a step against 176) and 1.2 times (128x128x64 in FP32, 194
+// against 162).
+int z_chunks(long tiles, int npz, long slots)
+{
+    int best = 1;
+    double least = 1e300;
+    for (int n = 1; n == 1 || n <= npz / 3; ++n) {
+        const double z = (double)npz / n;
+        if (z > 40.0 && n < npz / 3) continue;
+        const double w = (double)tiles * n / slots;
+        const double cost = (w <= 4.0 ? std::ceil(w) : w + 0.5) * (z + 0.7);
+        if (cost < least) {
+            least = cost;
+            best = n;
+        }
+    }
+    return best;
 }
 
 int create(const mhd3d_params* p, const double* const arrs[14], void** out)
@@ -1309,21 +1338,13 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
     s.plume = plume;
     std::free(hm);
 
-    // work decomposition: TX x TY tiles, z chunks of <= MHD3D_ZCHUNK planes;
-    // small grids take shorter chunks (>= 4 planes) so that the launch still
-    // fills about two waves of the SMs
+    // work decomposition: TX x TY tiles, z chunks by z_chunks()
     h->ntx = (npx + TX - 1) / TX;
     const int tyw = h->f32 ? TY32 : TY;
-    const long ntiles = (long)h->ntx * ((npy + tyw - 1) / tyw);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev);
-    const long want = 2L * sms * (h->f32 ? MHD3D_MINB32 : MHD3D_MINB);   // CTAs resident per SM
-    int nch = (npz + MHD3D_ZCHUNK - 1) / MHD3D_ZCHUNK;
-    const int fill = (int)std::min<long>((want + ntiles - 1) / ntiles, npz / 4);
-    if (fill > nch) nch = fill;
-    while (nch > 1 && npz / nch < 3) --nch;
-    h->nchunks = nch;
-    h->zlen = npz / nch;
+    h->nchunks = z_chunks((long)h->ntx * ((npy + tyw - 1) / tyw), npz,
+                          (long)sms * (h->f32 ? MHD3D_MINB32 : MHD3D_MINB));
 
     Control c0{};
     c0.timc = p->timc;
@@ -1897,10 +1918,9 @@ int ens_set_zlen(Ensemble* e, int zlen)
         const int npz = h->p.npz;
         int nch;
         if (zlen > 0) nch = std::max(1, npz / std::max(zlen, 3));
-        else nch = std::max(1, (npz + MHD3D_ZCHUNK - 1) / MHD3D_ZCHUNK);
+        else nch = (npz + 63) / 64;
         while (nch > 1 && npz / nch < 3) --nch;
         h->nchunks = nch;
-        h->zlen = npz / nch;
     }
     return ens_layout(e);
 }

@@ -30,9 +30,6 @@ namespace mhd3d {
 #ifndef MHD3D_TY
 #define MHD3D_TY 4
 #endif
-#ifndef MHD3D_ZCHUNK
-#define MHD3D_ZCHUNK 32           // planes a CTA marches through (z chunk length target)
-#endif
 constexpr int TX = 32;            // tile width (one warp per row)
 constexpr int TY = MHD3D_TY;      // tile rows (threads per CTA = 32*TY)
 constexpr int NT = TX * TY;       // threads per CTA
@@ -143,8 +140,7 @@ struct StageArgs {
     size_t zf, zz;          // Z: doubles per field, per plane
     int upitch, zpitch;
     int ntx;                // tiles along x
-    int zlen;               // planes per z chunk
-    int nchunks;
+    int nchunks;            // z chunks (chunk_start)
     long long wait_first;   // poll limit of a CTA's first ring wait (WAIT_LIMIT; lowered only by tests)
 };
 
@@ -225,8 +221,11 @@ struct StageArgs32 {
     float t_top_fix, t_top_fix4, t_top_flux, t_bot;   // wall T' constants (ITC 0/2/4, ITC=4 left half, ITC=1; IZC)
     size_t uf, uz, zf, zz;
     int upitch, zpitch;
-    int ntx, zlen, nchunks;
+    int ntx, nchunks;
 };
+
+// first plane of z chunk c of n: chunks differ by one plane at most
+__host__ __device__ inline int chunk_start(int c, int npz, int n) { return (int)((long long)c * npz / n); }
 
 // order-preserving map double -> uint64 and back
 __host__ __device__ inline unsigned long long key_of(double x)

@@ -170,8 +170,7 @@ __device__ __forceinline__ void stage32_item(const StageArgs32& a, const int til
     const int tid = threadIdx.x;
     const int tx = tid % TX, ty = tid / TX;
     const int x0 = (tile % a.ntx) * TX, y0 = (tile / a.ntx) * TYL;
-    const int k0 = chunk * a.zlen;
-    const int k1 = (chunk == a.nchunks - 1) ? npz : k0 + a.zlen;
+    const int k0 = chunk_start(chunk, npz, a.nchunks), k1 = chunk_start(chunk + 1, npz, a.nchunks);
     const int gi = x0 + tx, gj = y0 + ty;
     const bool active = gi < npx && gj < npy;
     const int lx = tx + BXO32, ly = ty + 1;

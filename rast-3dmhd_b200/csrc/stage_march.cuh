@@ -81,8 +81,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     const int tile = blockIdx.x;
     const int x0 = (tile % a.ntx) * TX, y0 = (tile / a.ntx) * TY;
     const int chunk = blockIdx.y;
-    const int k0 = chunk * a.zlen;
-    const int k1 = (chunk == a.nchunks - 1) ? npz : k0 + a.zlen;
+    const int k0 = chunk_start(chunk, npz, a.nchunks), k1 = chunk_start(chunk + 1, npz, a.nchunks);
     const int gi = x0 + tx, gj = y0 + ty;
     const bool active = gi < npx && gj < npy;
     const int o = (ty + 1) * BW + tx + BXO;   // own cell in a plane slot

@@ -101,33 +101,85 @@ struct Handle {
         }                                                                                        \
     } while (0)
 
-__global__ void k_unpack(const double* __restrict__ fort, double* __restrict__ u0, double* __restrict__ u1,
-                         int npx, int npy, int npz, int upitch, size_t uz)
+// ---- Fortran (NX,NY,NZ) arrays <-> the U layout --------------------------------
+// A warp walks a row of one field, four loads in flight a lane; a CTA takes
+// eight rows of a plane, blockIdx.y is the field of the list.  Bound by DRAM: upload
+// reads 8 and writes 8 (FP32: 4) bytes a value, download the reverse.  The
+// 1-D form with a division per element, writing both U buffers whole, ran at
+// 2.3 (FP64) and 3.1 TB/s (FP32) of these bytes.
+struct FieldList {
+    const double* src[8];
+    double* dst[8];
+    int fi[8];
+    int n;
+};
+constexpr int RW_ROWS = 8;   // rows a CTA
+
+dim3 rows_grid(int ny, int nz, int nfld) { return dim3((unsigned)(((ny + RW_ROWS - 1) / RW_ROWS) * nz), (unsigned)nfld); }
+
+// Halos are refreshed from the interior (COMMUNICATE's periodic copies),
+// ghost planes kept, in both buffers: a stage writes every other cell of its
+// output before anything reads it.  FP32 form: as perturbations from bg
+// (bg_row(fi) of 5 x NZ), rounded once.
+__host__ __device__ inline int bg_row(int f)
 {
-    // Fortran (NX,NY,NZ) -> both U buffers, halos refreshed from the interior
-    // (COMMUNICATE's periodic copies), ghost planes kept
+    return f == F_RO ? 0 : f == F_TT ? 1 : f == F_BX ? 2 : f == F_BY ? 3 : f == F_BZ ? 4 : -1;
+}
+template <typename T>
+__global__ void __launch_bounds__(32 * RW_ROWS) k_unpack(FieldList l, const double* __restrict__ bgd, T* __restrict__ u0,
+                                                         T* __restrict__ u1, int npx, int npy, int npz, int upitch,
+                                                         size_t uz, size_t uf, int cur)
+{
     const int NX = npx + 2, NY = npy + 2, NZ = npz + 2;
-    const size_t n = (size_t)NX * NY * NZ;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const int I = (int)(q % NX), J = (int)((q / NX) % NY), K = (int)(q / ((size_t)NX * NY));
-        const int Is = I == 0 ? npx : (I == NX - 1 ? 1 : I);
-        const int Js = J == 0 ? npy : (J == NY - 1 ? 1 : J);
-        const double v = fort[(size_t)Is + (size_t)NX * ((size_t)Js + (size_t)NY * K)];
-        const size_t d = (size_t)K * uz + (size_t)J * upitch + I;
-        u0[d] = v;
-        u1[d] = v;
+    const int nyb = (NY + RW_ROWS - 1) / RW_ROWS, f = blockIdx.y, fi = l.fi[f];
+    const int J = (blockIdx.x % nyb) * RW_ROWS + threadIdx.y, K = blockIdx.x / nyb;
+    if (J >= NY) return;
+    const int Js = J == 0 ? npy : (J == NY - 1 ? 1 : J);
+    const double* const s = l.src[f] + (size_t)NX * ((size_t)Js + (size_t)NY * K);
+    const size_t d = (size_t)fi * uf + (size_t)K * uz + (size_t)J * upitch;
+    T* const a = (cur ? u1 : u0) + d;
+    T* const b = (cur ? u0 : u1) + d;
+    const bool ghost = K == 0 || K == NZ - 1;
+    double bg = 0.0;
+    if (sizeof(T) == 4 && bg_row(fi) >= 0) bg = bgd[bg_row(fi) * NZ + K];
+    for (int I0 = threadIdx.x; I0 < NX; I0 += 128) {
+        double v[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int I = I0 + 32 * t, Is = I == 0 ? npx : (I == NX - 1 ? 1 : I);
+            v[t] = I < NX ? __ldcs(s + Is) : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int I = I0 + 32 * t;
+            if (I >= NX) continue;
+            const T x = (T)(sizeof(T) == 4 ? v[t] - bg : v[t]);
+            a[I] = x;
+            if (ghost) b[I] = x;
+        }
     }
 }
 
-__global__ void k_pack(const double* __restrict__ u, double* __restrict__ fort, int npx, int npy, int npz,
-                       int upitch, size_t uz)
+// U layout -> Fortran (NX,NY,NZ): the same index space, halos and ghost planes included
+template <typename T>
+__global__ void __launch_bounds__(32 * RW_ROWS) k_pack(FieldList l, const T* __restrict__ u, const double* __restrict__ bgd,
+                                                       int npx, int npy, int npz, int upitch, size_t uz, size_t uf)
 {
-    // U layout -> Fortran (NX,NY,NZ): the same index space, halos and ghost planes included
     const int NX = npx + 2, NY = npy + 2, NZ = npz + 2;
-    const size_t n = (size_t)NX * NY * NZ;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const int I = (int)(q % NX), J = (int)((q / NX) % NY), K = (int)(q / ((size_t)NX * NY));
-        fort[q] = u[(size_t)K * uz + (size_t)J * upitch + I];
+    const int nyb = (NY + RW_ROWS - 1) / RW_ROWS, f = blockIdx.y, fi = l.fi[f];
+    const int J = (blockIdx.x % nyb) * RW_ROWS + threadIdx.y, K = blockIdx.x / nyb;
+    if (J >= NY) return;
+    const T* const s = u + (size_t)fi * uf + (size_t)K * uz + (size_t)J * upitch;
+    double* const d = l.dst[f] + (size_t)NX * ((size_t)J + (size_t)NY * K);
+    const int br = sizeof(T) == 4 ? bg_row(fi) : -1;
+    const double bg = br >= 0 ? bgd[br * NZ + K] : 0.0;
+    for (int I0 = threadIdx.x; I0 < NX; I0 += 128) {
+        T v[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v[t] = I0 + 32 * t < NX ? s[I0 + 32 * t] : T(0);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (I0 + 32 * t < NX) __stcs(d + I0 + 32 * t, br >= 0 ? bg + (double)v[t] : (double)v[t]);
     }
 }
 
@@ -146,17 +198,39 @@ __global__ void k_pack_interior(const double* __restrict__ f, double* __restrict
     }
 }
 
-// horizontal mean of one Fortran (NX,NY,NZ) field per plane K over the
-// interior I=2..NX-1, J=2..NY-1, FP64, fixed summation order (one block per K)
-__global__ void k_hmean(const double* __restrict__ fort, double* __restrict__ mean, int npx, int npy)
+// horizontal means of Fortran (NX,NY,NZ) fields per plane K over the interior
+// I=2..NX-1, J=2..NY-1, FP64, fixed summation order: one block per plane and
+// field of the list (those with a background), eight loads in flight a thread
+__global__ void __launch_bounds__(256) k_hmean(FieldList l, double* __restrict__ bgd, int npx, int npy, int NZ)
 {
-    const int NX = npx + 2, NY = npy + 2;
-    const int K = blockIdx.x;
-    const double* pl = fort + (size_t)K * NX * NY;
+    const int br = bg_row(l.fi[blockIdx.y]);
+    if (br < 0) return;
+    const int NX = npx + 2, NY = npy + 2, K = blockIdx.x, n = npx * npy;
+    const double* pl = l.src[blockIdx.y] + (size_t)K * NX * NY + NX + 1;
+    const int di = 256 % npx, dj = 256 / npx;
+    int i = threadIdx.x % npx, j = threadIdx.x / npx;
     double acc = 0.0;
-    for (int q = threadIdx.x; q < npx * npy; q += blockDim.x) {
-        const int i = q % npx, j = q / npx;
-        acc += pl[(size_t)(j + 1) * NX + (i + 1)];
+    for (int q = threadIdx.x; q < n;) {
+        double v[8];
+        int m = 0;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            v[t] = 0.0;
+            if (q < n) {
+                v[t] = pl[(size_t)j * NX + i];
+                m = t + 1;
+            }
+            q += 256;
+            i += di;
+            j += dj;
+            if (i >= npx) {
+                i -= npx;
+                ++j;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            if (t < m) acc += v[t];
     }
     __shared__ double red[256];
     red[threadIdx.x] = acc;
@@ -165,39 +239,7 @@ __global__ void k_hmean(const double* __restrict__ fort, double* __restrict__ me
         if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) mean[K] = red[0] / ((double)npx * (double)npy);
-}
-
-// Fortran (NX,NY,NZ) FP64 -> both FP32 U buffers as perturbations from bg(K)
-// (bg may be null: no background), halos refreshed from the interior
-__global__ void k_unpack32(const double* __restrict__ fort, const double* __restrict__ bg, float* __restrict__ u0,
-                           float* __restrict__ u1, int npx, int npy, int npz, int upitch, size_t uz)
-{
-    const int NX = npx + 2, NY = npy + 2, NZ = npz + 2;
-    const size_t n = (size_t)NX * NY * NZ;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const int I = (int)(q % NX), J = (int)((q / NX) % NY), K = (int)(q / ((size_t)NX * NY));
-        const int Is = I == 0 ? npx : (I == NX - 1 ? 1 : I);
-        const int Js = J == 0 ? npy : (J == NY - 1 ? 1 : J);
-        double v = fort[(size_t)Is + (size_t)NX * ((size_t)Js + (size_t)NY * K)];
-        if (bg) v -= bg[K];
-        const size_t d = (size_t)K * uz + (size_t)J * upitch + I;
-        u0[d] = (float)v;
-        u1[d] = (float)v;
-    }
-}
-
-// FP32 U layout -> Fortran (NX,NY,NZ) FP64 full values
-__global__ void k_pack32(const float* __restrict__ u, const double* __restrict__ bg, double* __restrict__ fort,
-                         int npx, int npy, int npz, int upitch, size_t uz)
-{
-    const int NX = npx + 2, NY = npy + 2, NZ = npz + 2;
-    const size_t n = (size_t)NX * NY * NZ;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const int I = (int)(q % NX), J = (int)((q / NX) % NY), K = (int)(q / ((size_t)NX * NY));
-        const double v = (double)u[(size_t)K * uz + (size_t)J * upitch + I];
-        fort[q] = bg ? bg[K] + v : v;
-    }
+    if (threadIdx.x == 0) bgd[(size_t)br * NZ + K] = red[0] / ((double)npx * (double)npy);
 }
 
 // FP32 Z layout (interior) -> Fortran (NX,NY,NZ) FP64, zeros outside
@@ -246,7 +288,7 @@ __global__ void __launch_bounds__(PROF_THREADS) k_profiles(const void* __restric
     auto val = [&](int f, size_t off) -> double {
         if (F32) {
             const double v = (double)reinterpret_cast<const float*>(ubuf)[(size_t)f * uf + off];
-            const int bi = f == F_RO ? 0 : f == F_TT ? 1 : f == F_BX ? 2 : f == F_BY ? 3 : f == F_BZ ? 4 : -1;
+            const int bi = bg_row(f);
             return bi >= 0 ? bgd[bi * NZ + K0] + v : v;
         }
         return reinterpret_cast<const double*>(ubuf)[(size_t)f * uf + off];
@@ -338,7 +380,7 @@ __device__ __forceinline__ double uget(const UView& v, int f, int i, int j, int 
     const size_t off = (size_t)f * v.uf + (size_t)K * v.uz + (size_t)j * v.upitch + i;
     if (v.f32) {
         const double x = (double)static_cast<const float*>(v.u)[off];
-        const int bi = f == F_RO ? 0 : f == F_TT ? 1 : f == F_BX ? 2 : f == F_BY ? 3 : f == F_BZ ? 4 : -1;
+        const int bi = bg_row(f);
         return bi >= 0 ? v.bgd[bi * v.NZ + K] + x : x;
     }
     return static_cast<const double*>(v.u)[off];
@@ -1358,19 +1400,6 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
     return MHD3D_OK;
 }
 
-// background index of a field in the FP32 form (-1: stored whole)
-int bg_index(int fi)
-{
-    switch (fi) {
-        case F_RO: return 0;
-        case F_TT: return 1;
-        case F_BX: return 2;
-        case F_BY: return 3;
-        case F_BZ: return 4;
-        default: return -1;
-    }
-}
-
 // FP32 form: per-plane background terms from the FP64 horizontal means
 int set_background(Handle* h)
 {
@@ -1445,41 +1474,91 @@ int set_background(Handle* h)
     return MHD3D_OK;
 }
 
-// Upload and download move one field at a time through two staging fields:
-// the copy of field i (on the copy stream) overlaps the unpack or pack of
-// field i-1 (on the handle's stream); events order each staging field's
-// copy, kernel and reuse two fields later.
+// Whether the field arrays can be read or written by kernels in place: memory
+// of the handle's device, on 8 bytes, no two arrays overlapping (a copy through
+// the staging fields takes them in order).
+bool in_place(const Handle* h, const void* const f[8], size_t bytes)
+{
+    for (int i = 0; i < h->nf; ++i) {
+        if (!f[i]) continue;
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, f[i]) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeDevice || at.device != h->dev || (reinterpret_cast<uintptr_t>(f[i]) & 7u)) return false;
+        for (int j = 0; j < i; ++j) {
+            const char *x = static_cast<const char*>(f[i]), *y = static_cast<const char*>(f[j]);
+            if (y && x < y + bytes && y < x + bytes) return false;
+        }
+    }
+    return true;
+}
+
+cudaError_t unpack_fields(Handle* h, const FieldList& l)
+{
+    const int npx = h->p.npx, npy = h->p.npy, npz = h->p.npz;
+    const dim3 g = rows_grid(npy + 2, npz + 2, l.n), b(32, RW_ROWS);
+    if (h->f32) {
+        k_hmean<<<dim3((unsigned)(npz + 2), (unsigned)l.n), 256, 0, h->st>>>(l, h->bgd, npx, npy, npz + 2);
+        k_unpack<float><<<g, b, 0, h->st>>>(l, h->bgd, reinterpret_cast<float*>(h->ubuf[0]),
+                                           reinterpret_cast<float*>(h->ubuf[1]), npx, npy, npz, h->upitch, h->uz, h->uf,
+                                           h->cur);
+    } else {
+        k_unpack<double><<<g, b, 0, h->st>>>(l, nullptr, h->ubuf[0], h->ubuf[1], npx, npy, npz, h->upitch, h->uz, h->uf,
+                                            h->cur);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t pack_fields(Handle* h, const FieldList& l)
+{
+    const int npx = h->p.npx, npy = h->p.npy, npz = h->p.npz;
+    const dim3 g = rows_grid(npy + 2, npz + 2, l.n), b(32, RW_ROWS);
+    if (h->f32)
+        k_pack<float><<<g, b, 0, h->st>>>(l, reinterpret_cast<const float*>(h->ubuf[h->cur]), h->bgd, npx, npy, npz,
+                                         h->upitch, h->uz, h->uf);
+    else k_pack<double><<<g, b, 0, h->st>>>(l, h->ubuf[h->cur], nullptr, npx, npy, npz, h->upitch, h->uz, h->uf);
+    return cudaGetLastError();
+}
+
+// Upload and download: arrays in device memory are read and written by the
+// kernels in place, all fields in one launch.  Others move one field at a time
+// through two staging fields: the copy of field i (on the copy stream)
+// overlaps the unpack or pack of field i-1 (on the handle's stream); events
+// order each staging field's copy, kernel and reuse two fields later.
 int upload(Handle* h, const double* const f[8])
 {
     CK(cudaSetDevice(h->dev));
-    const int npx = h->p.npx, npy = h->p.npy, npz = h->p.npz;
-    const size_t nfort = (size_t)(npx + 2) * (npy + 2) * (npz + 2);
+    const size_t nfort = (size_t)(h->p.npx + 2) * (h->p.npy + 2) * (h->p.npz + 2);
     for (int i = 0; i < h->nf; ++i)
         if (!f[i]) return MHD3D_ERR_ARG;
-    // the staging fields are free once the handle's stream has drained
-    CK(cudaEventRecord(h->ev_kern[1], h->st));
-    CK(cudaStreamWaitEvent(h->cst, h->ev_kern[1], 0));
-    for (int fi = 0; fi < h->nf; ++fi) {
-        const int b = fi & 1;
-        double* const stg = b ? h->stage2 : h->stage;
-        if (fi >= 2) CK(cudaStreamWaitEvent(h->cst, h->ev_kern[b], 0));   // field fi-2 unpacked
-        CK(cudaMemcpyAsync(stg, f[fi], sizeof(double) * nfort, cudaMemcpyDefault, h->cst));
-        CK(cudaEventRecord(h->ev_copy[b], h->cst));
-        CK(cudaStreamWaitEvent(h->st, h->ev_copy[b], 0));
-        if (h->f32) {
-            const int bi = bg_index(fi);
-            double* bg = bi >= 0 ? h->bgd + (size_t)bi * (npz + 2) : nullptr;
-            if (bg) k_hmean<<<npz + 2, 256, 0, h->st>>>(stg, bg, npx, npy);
-            float* u0 = reinterpret_cast<float*>(h->ubuf[0]) + (size_t)fi * h->uf;
-            float* u1 = reinterpret_cast<float*>(h->ubuf[1]) + (size_t)fi * h->uf;
-            k_unpack32<<<grid_for(nfort), 256, 0, h->st>>>(stg, bg, u0, u1, npx, npy, npz, h->upitch, h->uz);
-        } else {
-            k_unpack<<<grid_for(nfort), 256, 0, h->st>>>(stg, h->ubuf[0] + (size_t)fi * h->uf,
-                                                         h->ubuf[1] + (size_t)fi * h->uf, npx, npy, npz, h->upitch,
-                                                         h->uz);
+    if (in_place(h, reinterpret_cast<const void* const*>(f), sizeof(double) * nfort)) {
+        FieldList l{};
+        for (int fi = 0; fi < h->nf; ++fi) {
+            l.src[fi] = f[fi];
+            l.fi[fi] = fi;
         }
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(h->ev_kern[b], h->st));
+        l.n = h->nf;
+        CK(unpack_fields(h, l));
+    } else {
+        // the staging fields are free once the handle's stream has drained
+        CK(cudaEventRecord(h->ev_kern[1], h->st));
+        CK(cudaStreamWaitEvent(h->cst, h->ev_kern[1], 0));
+        for (int fi = 0; fi < h->nf; ++fi) {
+            const int b = fi & 1;
+            double* const stg = b ? h->stage2 : h->stage;
+            if (fi >= 2) CK(cudaStreamWaitEvent(h->cst, h->ev_kern[b], 0));   // field fi-2 unpacked
+            CK(cudaMemcpyAsync(stg, f[fi], sizeof(double) * nfort, cudaMemcpyDefault, h->cst));
+            CK(cudaEventRecord(h->ev_copy[b], h->cst));
+            CK(cudaStreamWaitEvent(h->st, h->ev_copy[b], 0));
+            FieldList l{};
+            l.src[0] = stg;
+            l.fi[0] = fi;
+            l.n = 1;
+            CK(unpack_fields(h, l));
+            CK(cudaEventRecord(h->ev_kern[b], h->st));
+        }
     }
     CK(cudaStreamSynchronize(h->st));
     if (h->f32) {
@@ -1495,31 +1574,35 @@ int upload(Handle* h, const double* const f[8])
 int download(Handle* h, double* const f[8])
 {
     CK(cudaSetDevice(h->dev));
-    const int npx = h->p.npx, npy = h->p.npy, npz = h->p.npz;
-    const size_t nfort = (size_t)(npx + 2) * (npy + 2) * (npz + 2);
-    int n = 0;
-    for (int fi = 0; fi < h->nf; ++fi) {
-        if (!f[fi]) continue;
-        const int b = n & 1;
-        double* const stg = b ? h->stage2 : h->stage;
-        if (n >= 2) CK(cudaStreamWaitEvent(h->st, h->ev_copy[b], 0));   // the copy of two fields ago done
-        if (h->f32) {
-            const int bi = bg_index(fi);
-            k_pack32<<<grid_for(nfort), 256, 0, h->st>>>(
-                reinterpret_cast<const float*>(h->ubuf[h->cur]) + (size_t)fi * h->uf,
-                bi >= 0 ? h->bgd + (size_t)bi * (npz + 2) : nullptr, stg, npx, npy, npz, h->upitch, h->uz);
-        } else {
-            k_pack<<<grid_for(nfort), 256, 0, h->st>>>(h->ubuf[h->cur] + (size_t)fi * h->uf, stg, npx, npy,
-                                                       npz, h->upitch, h->uz);
+    const size_t nfort = (size_t)(h->p.npx + 2) * (h->p.npy + 2) * (h->p.npz + 2);
+    if (in_place(h, reinterpret_cast<const void* const*>(f), sizeof(double) * nfort)) {
+        FieldList l{};
+        for (int fi = 0; fi < h->nf; ++fi) {
+            if (!f[fi]) continue;
+            l.dst[l.n] = f[fi];
+            l.fi[l.n++] = fi;
         }
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(h->ev_kern[b], h->st));
-        CK(cudaStreamWaitEvent(h->cst, h->ev_kern[b], 0));
-        CK(cudaMemcpyAsync(f[fi], stg, sizeof(double) * nfort, cudaMemcpyDefault, h->cst));
-        CK(cudaEventRecord(h->ev_copy[b], h->cst));
-        ++n;
+        if (l.n) CK(pack_fields(h, l));
+    } else {
+        int n = 0;
+        for (int fi = 0; fi < h->nf; ++fi) {
+            if (!f[fi]) continue;
+            const int b = n & 1;
+            double* const stg = b ? h->stage2 : h->stage;
+            if (n >= 2) CK(cudaStreamWaitEvent(h->st, h->ev_copy[b], 0));   // the copy of two fields ago done
+            FieldList l{};
+            l.dst[0] = stg;
+            l.fi[0] = fi;
+            l.n = 1;
+            CK(pack_fields(h, l));
+            CK(cudaEventRecord(h->ev_kern[b], h->st));
+            CK(cudaStreamWaitEvent(h->cst, h->ev_kern[b], 0));
+            CK(cudaMemcpyAsync(f[fi], stg, sizeof(double) * nfort, cudaMemcpyDefault, h->cst));
+            CK(cudaEventRecord(h->ev_copy[b], h->cst));
+            ++n;
+        }
+        CK(cudaStreamSynchronize(h->cst));
     }
-    CK(cudaStreamSynchronize(h->cst));
     CK(cudaStreamSynchronize(h->st));
     return MHD3D_OK;
 }

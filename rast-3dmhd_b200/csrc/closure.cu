@@ -26,10 +26,9 @@
 //    below, and writes BF16 (and FP32) outputs.
 //  - k_conv3d_wgrad_tc: dW[n][tap*CIN+ci] = sum over voxels of dY[v][n] *
 //    X[v+tap][ci] on tcgen05 as well, with K running over voxels: per x
-//    segment the shifted dY rows form A (M = 3*COUT, the x taps) and the
-//    input rows of the y taps form B (N = 3*CIN, the z taps), both staged
-//    K-major by the CTA's threads; per-CTA partials are added in CTA order
-//    by k_wgrad_reduce.
+//    segment a dY row read at the three x shifts forms A and the input rows
+//    of the y taps form B (the z taps), both MN-major as they lie in memory;
+//    per-CTA partials are added in CTA order by k_wgrad_reduce.
 //
 // Every wait is bounded; a CTA that gives up records an error and releases
 // its tensor memory.
@@ -604,86 +603,110 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
 // (x0..x0+63) of one (y, z) row, with u = 0..KT-1 indexing x0-1+u:
 //
 //   A[(dx, n)][u]   = dY[x0 + u - dx][n]  (zero outside the segment's own
-//                     voxels; rows 3*COUT..127 zero)           M = 128
+//                     voxels)                              M = 128
 //   B_dy[(dz,ci)][u] = X[x0-1+u, y+dy-1, z+dz-1][ci] (periodic in x, y; zero
 //                     outside z and for u >= WT+2)             N = 3*CIN
 //   D_dy[(dx,n)][(dz,ci)] += sum_u A B_dy                      K = KT = 80
 //
-// so one segment is 3 (y taps) x 5 (K steps of 16) MMAs of M=128, N=3*CIN,
-// both operands K-major in the canonical no-swizzle layout, staged by the
-// CTA's threads: A from a transposed copy of the segment's dY (the x tap is
-// a shift by 0..2 elements, formed with byte permutes), B by 8x8 transposes
-// of the channels-last input.  Segments alternate between two staging
-// buffers, so the MMAs of one overlap the staging of the next.  The three
-// accumulators (3*3*CIN columns) stay in TMEM over all of a CTA's segments
-// (a fixed set, in a fixed order); each CTA writes its partial sums to a
-// workspace row and a second kernel adds the rows to dW in CTA order, so the
-// result does not depend on timing.
+// so one segment is 3 (y taps) x 5 (K steps of 16) MMAs of M=128, N=3*CIN.
+// Channels-last rows are MN-major operands as they lie in memory: a voxel is
+// one row of K, its channels one row of M or N (64- or 32-byte rows in the
+// swizzle of that width, which the matrix descriptors read back), so TMA boxes
+// of 64 voxels (x a multiple of 64; the two halo voxels, and any other row, by
+// cp.async) fill both operands and nothing is transposed.  The x taps are blocks of one
+// staged dY row that start a voxel apart (block j holds dx = 2-j; the leading
+// offset of A is one voxel; blocks beyond the third are unused lanes), the z
+// taps the three planes of an input row.  The loader warps run up to WST
+// segments ahead of the MMA thread.  The three accumulators (3*3*CIN columns)
+// stay in TMEM over all of a CTA's segments (a fixed set, in a fixed order);
+// each CTA writes its partial sums to a workspace row and a second kernel adds
+// the rows to dW in CTA order, so the result does not depend on timing.
+//
+// Bound by L2 reads (42 KB a segment for 32 input channels) and the hand-offs
+// of three stages; 128x128x64, us: 16->32 117, 32->32 143, 32->16 129.  The
+// form that transposed both operands through registers took 463, 657 and 605,
+// this one with every row by cp.async 151, 241 and 231.  Marching along y with
+// 128-voxel segments and the roles of the operands exchanged took 137, 146 and
+// 114, but sums in another order; this one's bits are those of the first form.
 constexpr int WT = 64;               // voxels of an x segment
 constexpr int KT = 80;               // K of a segment: WT + 2 halo voxels, padded to 16
-constexpr int WG_NTH = 256;          // threads of a weight-gradient CTA
-constexpr int DYW = 8 + KT + 8;      // row of the transposed dY: 8 zeros, the segment, zeros
+constexpr int WG_LD = 8;             // loader warps
+constexpr int WG_SUM = 256;          // threads that sum dY (the first four warps are the epilogue)
+constexpr int WG_NTH = WG_SUM + 32 * (WG_LD + 1);
+// Rows of the staged operands: voxel x0 of an input row or of dY sits at row 8,
+// a TMA destination (512 or 256 bytes); u = 0 is row WXR0 of an input row and
+// row WYR0 of dY with dx = 2.
+constexpr int WXR0 = 7, WYR0 = 6;
+constexpr int WXR = 88;              // rows of an input row: WXR0 + KT rounded up to 8
+constexpr int WYR = 96;              // of dY: WYR0 + KT and what the unused blocks read
+constexpr int WST = 3;               // stages
 
 template <int CIN, int COUT>
 struct WgLay {
+    static constexpr int XB = CIN * 2, YB = COUT * 2;         // bytes of a voxel
     static constexpr int N = 3 * CIN;                         // columns of one y-tap accumulator
     static constexpr uint32_t NCOL = 3 * N <= 256 ? 256 : 512;
-    static constexpr size_t A_B = (size_t)(KT / 8) * 128 * 16;    // one A buffer
-    static constexpr size_t BD_B = (size_t)(KT / 8) * N * 16;     // one y tap of a B buffer
-    static constexpr size_t B_B = 3 * BD_B;
-    static constexpr size_t BUF_B = A_B + B_B;
-    static constexpr size_t DYT_OFF = 2 * BUF_B;
-    static constexpr size_t DYT_B = (size_t)COUT * DYW * 2;
-    static constexpr size_t RED_OFF = (DYT_OFF + DYT_B + 15) / 16 * 16;
-    static constexpr size_t RED_B = (size_t)WG_NTH * 8 * 4;
-    static constexpr size_t BAR_OFF = RED_OFF + RED_B;
-    static constexpr size_t BYTES = BAR_OFF + 2 * 8 + 16 + 1024;   // + alignment of the base to 1024 bytes
+    static constexpr int X_ROW = WXR * XB;                    // one input row (y, z)
+    static constexpr int Y_OFF = (9 * X_ROW + 511) / 512 * 512;   // dY behind the nine input rows of a stage
+    static constexpr int STAGE_B = (Y_OFF + WYR * YB + 1023) / 1024 * 1024;
+    static constexpr int RED_OFF = WST * STAGE_B;
+    static constexpr int BAR_OFF = RED_OFF + WG_SUM * 8 * 4;
+    // barriers: ready[WST], mmadone[WST], sumdone[WST]; the TMEM address, the
+    // abort flag and the last committed segment
+    static constexpr size_t BYTES = BAR_OFF + 3 * WST * 8 + 16 + 1024;   // + alignment of the base to 1024 bytes
 };
 
-// 8x8 transpose of BF16: v[a] holds 8 channels of voxel a (word w: channels
-// 2w, 2w+1); r[i] receives voxels 0..7 of channel i
-__device__ __forceinline__ void transpose8(const uint4 (&v)[8], uint4 (&r)[8])
+// matrix descriptor of an MN-major operand: rows of ROWB bytes (64: 64-byte
+// swizzle, 32: 32-byte swizzle) along K, 8-row groups ROWB*8 bytes apart,
+// blocks of ROWB bytes along MN lbo bytes apart
+template <int ROWB>
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t lbo)
 {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
-        uint32_t o[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const uint4& a = v[2 * w];
-            const uint4& b = v[2 * w + 1];
-            const uint32_t wa = (i >> 1) == 0 ? a.x : (i >> 1) == 1 ? a.y : (i >> 1) == 2 ? a.z : a.w;
-            const uint32_t wb = (i >> 1) == 0 ? b.x : (i >> 1) == 1 ? b.y : (i >> 1) == 2 ? b.z : b.w;
-            o[w] = __byte_perm(wa, wb, sel);
-        }
-        r[i] = make_uint4(o[0], o[1], o[2], o[3]);
-    }
+    uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)(ROWB * 8 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)(ROWB == 64 ? 4 : 6) << 61;
+    return d;
+}
+
+// 16-byte chunk c of row r of an operand whose rows have ROWB bytes
+template <int ROWB>
+__device__ __forceinline__ uint32_t swz_chunk(int r, int c)
+{
+    return (uint32_t)(r * ROWB + ((ROWB == 64 ? c ^ ((r >> 1) & 3) : c ^ ((r >> 2) & 1)) * 16));
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool on)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16u : 0u) : "memory");
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
+                                                               const __grid_constant__ CUtensorMap ymap, int use_tma,
+                                                               const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ dy,
                                                                float* __restrict__ ws, int nx, int ny, int nz,
                                                                int* __restrict__ err)
 {
     using L = WgLay<CIN, COUT>;
-    constexpr int N = L::N, K = 27 * CIN, NCC = CIN / 8, NNC = COUT / 8;
+    constexpr int N = L::N, K = 27 * CIN, NCX = CIN / 8, NCY = COUT / 8;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* const sb = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    __nv_bfloat16* const dyt = reinterpret_cast<__nv_bfloat16*>(sb + L::DYT_OFF);
+    const uint32_t sa = smem_u32(sb);
     float* const red = reinterpret_cast<float*>(sb + L::RED_OFF);
-    unsigned long long* const mmadone = reinterpret_cast<unsigned long long*>(sb + L::BAR_OFF);
-    uint32_t* const tslot = reinterpret_cast<uint32_t*>(sb + L::BAR_OFF + 16);
-    volatile int* const abort_flag = reinterpret_cast<volatile int*>(sb + L::BAR_OFF + 20);
+    unsigned long long* const ready = reinterpret_cast<unsigned long long*>(sb + L::BAR_OFF);
+    unsigned long long* const mmadone = ready + WST;
+    unsigned long long* const sumdone = ready + 2 * WST;
+    uint32_t* const tslot = reinterpret_cast<uint32_t*>(sb + L::BAR_OFF + 3 * WST * 8);
+    volatile int* const abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
+    volatile int* const last_commit = reinterpret_cast<volatile int*>(tslot + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // A rows 3*COUT..127 stay zero in both buffers; the dY padding is rewritten per segment
-    for (int q = tid; q < 2 * (KT / 8) * 128; q += WG_NTH) {
-        const int b = q / ((KT / 8) * 128), r = q % ((KT / 8) * 128);
-        const int row = r % 128, kc = r / 128;
-        if (row >= 3 * COUT)
-            *reinterpret_cast<uint4*>(sb + b * L::BUF_B + (size_t)kc * 2048 + row * 16) = make_uint4(0, 0, 0, 0);
-    }
+    // what no copy writes stays zero: input rows u >= WT+2, dY outside the segment
+    for (int q = tid; q < WST * L::STAGE_B / 16; q += WG_NTH)
+        *reinterpret_cast<uint4*>(sb + (size_t)q * 16) = make_uint4(0, 0, 0, 0);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                      "r"(L::NCOL)
@@ -691,11 +714,16 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __nv_bfloat
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(mmadone + 0, 1);
-        mbar_init(mmadone + 1, 1);
+        for (int b = 0; b < WST; ++b) {
+            mbar_init(ready + b, use_tma ? 1 + 32 : 32 * WG_LD);
+            mbar_init(mmadone + b, 1);
+            mbar_init(sumdone + b, WG_SUM / 32);
+        }
         *abort_flag = 0;
+        *last_commit = -1;
         fence_mbar_init();
     }
+    fence_proxy_async();   // the zeros, written by plain stores, are read by the tensor cores
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -703,147 +731,166 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __nv_bfloat
 
     const int nseg = (nx + WT - 1) / WT;
     const int ntile = nseg * ny * nz;
-    float dbacc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // dY sums of this thread's 8 channels
-    int i = 0;
-    for (int t = blockIdx.x; t < ntile; t += gridDim.x, ++i) {
-        const int seg = t % nseg, yy = (t / nseg) % ny, zz = t / (nseg * ny);
-        const int x0 = seg * WT;
-        const int mlim = nx - x0 < WT ? nx - x0 : WT;   // the segment's own voxels (nx < 64: one period)
-        const int b = i & 1;
-        unsigned char* const sa = sb + b * L::BUF_B;
-        unsigned char* const sbb = sa + L::A_B;
-        // the buffer was last read by the MMAs of segment i-2
-        if (i >= 2) {
-            bool ok = true;
-            if (tid == 0) ok = mbar_wait(mmadone + b, (unsigned)((i - 2) >> 1) & 1u);
-            if (!ok) *abort_flag = 1;
+    // segments blockIdx.x, blockIdx.x + gridDim.x, ..: the i-th in stage i % WST;
+    // f(i, t, stage, parity) returns false to stop
+    auto segments = [&](auto f) {
+        int i = 0, st = 0;
+        unsigned ph = 0;
+        for (int t = blockIdx.x; t < ntile; t += gridDim.x, ++i) {
+            if (*abort_flag || !f(i, t, st, ph)) return;
+            if (++st == WST) {
+                st = 0;
+                ph ^= 1u;
+            }
         }
-        __syncthreads();
-        if (*abort_flag) break;
-        // ---- dY of the segment, transposed: dyt[n][8 + j], zeros around it
-        {
-            const size_t row = ((size_t)zz * ny + yy) * nx + x0;
-            for (int q = tid; q < WT * NNC; q += WG_NTH) {
-                const int nc = q % NNC, j = q / NNC;
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (j < mlim) v = __ldg(reinterpret_cast<const uint4*>(dy + (row + j) * COUT + nc * 8));
+    };
+    auto give_up = [&]() {
+        *abort_flag = 1;
+        atomicExch(err, 1);
+        return false;
+    };
+
+    float dbacc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // dY sums of this thread's 8 channels
+    if (use_tma && warp == WG_SUM / 32) {
+        // one warp: ten TMA boxes and the input rows' halo voxels
+        segments([&](int i, int t, int st, unsigned ph) {
+            if (i >= WST && (!mbar_wait_fast(mmadone + st, ph ^ 1u) || !mbar_wait_fast(sumdone + st, ph ^ 1u)))
+                return give_up();
+            const int x0 = (t % nseg) * WT, yy = (t / nseg) % ny, zz = t / (nseg * ny);
+            const uint32_t sx = sa + (uint32_t)(st * L::STAGE_B);
+            if (lane == 0) {
+                mbar_expect_tx(ready + st, (unsigned)(9 * WT * L::XB + WT * L::YB));
+                for (int rz = 0; rz < 9; ++rz) {
+                    int gy = yy + rz / 3 - 1;
+                    gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
+                    tma_load4(sb + (size_t)st * L::STAGE_B + rz * L::X_ROW + 8 * L::XB, &xmap, ready + st, 0, x0, gy,
+                              zz + rz % 3 - 1);   // zeros outside z
+                }
+                tma_load4(sb + (size_t)st * L::STAGE_B + L::Y_OFF + 8 * L::YB, &ymap, ready + st, 0, x0, yy, zz);
+            }
+            for (int q = lane; q < 9 * 2 * NCX; q += 32) {
+                const int c = q % NCX, side = q / NCX % 2, rz = q / (2 * NCX);
+                int gy = yy + rz / 3 - 1;
+                gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
+                const int gz = zz + rz % 3 - 1;
+                const bool on = gz >= 0 && gz < nz;
+                int gx = side ? x0 + WT : x0 - 1;
+                gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
+                cp_async16(sx + (uint32_t)(rz * L::X_ROW) + swz_chunk<L::XB>(side ? 8 + WT : 7, c),
+                           x + (((size_t)(on ? gz : zz) * ny + gy) * nx + gx) * CIN + c * 8, on);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(ready + st)) : "memory");
+            return true;
+        });
+        cp_async_wait<0>();
+    } else if (!use_tma && tid >= WG_SUM && warp < WG_SUM / 32 + WG_LD) {
+        const int lt = tid - WG_SUM;
+        segments([&](int i, int t, int st, unsigned ph) {
+            // the stage was last read by the segment WST before
+            if (i >= WST && (!mbar_wait_fast(mmadone + st, ph ^ 1u) || !mbar_wait_fast(sumdone + st, ph ^ 1u)))
+                return give_up();
+            const int x0 = (t % nseg) * WT, yy = (t / nseg) % ny, zz = t / (nseg * ny);
+            const uint32_t sx = sa + (uint32_t)(st * L::STAGE_B), sy = sx + L::Y_OFF;
+            const __nv_bfloat16* const drow = dy + (((size_t)zz * ny + yy) * nx + x0) * COUT;
+            const int mlim = nx - x0 < WT ? nx - x0 : WT;   // the segment's own voxels (nx < 64: one period)
+            for (int q = lt; q < WT * NCY; q += 32 * WG_LD) {
+                const int c = q % NCY, j = q / NCY;
+                cp_async16(sy + swz_chunk<L::YB>(j + 8, c), drow + (size_t)(j < mlim ? j : 0) * COUT + c * 8, j < mlim);
+            }
+            // a (row, voxel) pair a step of the loop: its chunks by adjacent threads
+            constexpr int RP = 32 * WG_LD / NCX;   // pairs in flight over the loaders
+            const int c = lt % NCX;
+            for (int q = lt / NCX; q < 9 * (WT + 2); q += RP) {
+                const int rz = q / (WT + 2), u = q % (WT + 2);
+                int gy = yy + rz / 3 - 1;
+                gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
+                const int gz = zz + rz % 3 - 1;
+                const bool on = gz >= 0 && gz < nz;
+                int gx = x0 - 1 + u;
+                if (nx >= WT) gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
+                else gx = (gx + nx) % nx;
+                cp_async16(sx + (uint32_t)(rz * L::X_ROW) + swz_chunk<L::XB>(WXR0 + u, c),
+                           x + (((size_t)(on ? gz : zz) * ny + gy) * nx + gx) * CIN + c * 8, on);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(ready + st)) : "memory");
+            return true;
+        });
+        cp_async_wait<0>();
+    } else if (warp == WG_SUM / 32 + WG_LD) {
+        if (lane == 0) {
+            constexpr uint32_t IDESC = idesc_bf16(128, N) | (1u << 15) | (1u << 16);   // both operands MN-major
+            segments([&](int i, int, int st, unsigned ph) {
+                if (!mbar_wait_fast(ready + st, ph)) return give_up();
+                fence_proxy_async();   // rows written by cp.async are read by the tensor cores
+                tc_fence_after();
+                const uint32_t sx = sa + (uint32_t)(st * L::STAGE_B);
+                const uint64_t da = smem_desc_mn<L::YB>(sx + L::Y_OFF + WYR0 * L::YB, L::YB);
+                const uint64_t db = smem_desc_mn<L::XB>(sx + WXR0 * L::XB, L::X_ROW);
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int k2 = 0; k2 < KT / 16; ++k2)
+                        umma_bf16(tmem + (uint32_t)(d * N), da + (uint64_t)(k2 * L::YB),
+                                  db + (uint64_t)((d * 3 * L::X_ROW >> 4) + k2 * L::XB), IDESC,
+                                  (i == 0 && k2 == 0) ? 0u : 1u);
+                umma_commit(mmadone + st);
+                *last_commit = i;
+                return true;
+            });
+        }
+        __syncwarp();
+    } else if (tid < WG_SUM) {
+        // bias gradient from the staged dY (zeros beyond the segment's own voxels)
+        segments([&](int, int, int st, unsigned ph) {
+            if (!mbar_wait_fast(ready + st, ph)) return give_up();
+            const unsigned char* const sy = sb + (size_t)st * L::STAGE_B + L::Y_OFF;
+            for (int q = tid; q < WT * NCY; q += WG_SUM) {
+                const uint4 v = *reinterpret_cast<const uint4*>(sy + swz_chunk<L::YB>(q / NCY + 8, q % NCY));
                 const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&v);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    dyt[(nc * 8 + e) * DYW + 8 + j] = h[e];
-                    dbacc[e] += __bfloat162float(h[e]);
-                }
+                for (int e = 0; e < 8; ++e) dbacc[e] += __bfloat162float(h[e]);
             }
-            for (int q = tid; q < COUT * 16; q += WG_NTH) {
-                const int n = q / 16, e = q % 16;
-                dyt[n * DYW + (e < 8 ? e : 8 + WT + (e - 8))] = __float2bfloat16_rn(0.f);
-            }
-            for (int q = tid; q < COUT * (KT - WT); q += WG_NTH) {   // beyond the segment up to KT
-                const int n = q / (KT - WT), e = q % (KT - WT);
-                if (8 + WT + 8 + e < DYW) dyt[n * DYW + 8 + WT + 8 + e] = __float2bfloat16_rn(0.f);
-            }
-        }
-        __syncthreads();
-        // ---- A[(dx, n)][u] = dyt[n][8 + u - dx]: 16-byte rows (kc, row)
-        for (int q = tid; q < (KT / 8) * 3 * COUT; q += WG_NTH) {
-            const int kc = q / (3 * COUT), m = q % (3 * COUT);
-            const int dxs = m / COUT, n = m % COUT;
-            const uint4 c0 = *reinterpret_cast<const uint4*>(dyt + n * DYW + kc * 8);       // elements 8kc-8 ..
-            const uint4 c1 = *reinterpret_cast<const uint4*>(dyt + n * DYW + kc * 8 + 8);   // elements 8kc ..
-            uint4 o;
-            if (dxs == 0) o = c1;
-            else if (dxs == 2) o = make_uint4(c0.w, c1.x, c1.y, c1.z);
-            else o = make_uint4(__byte_perm(c0.w, c1.x, 0x5432), __byte_perm(c1.x, c1.y, 0x5432),
-                                __byte_perm(c1.y, c1.z, 0x5432), __byte_perm(c1.z, c1.w, 0x5432));
-            *reinterpret_cast<uint4*>(sa + (size_t)kc * 2048 + m * 16) = o;
-        }
-        // ---- B_dy[(dz, ci)][u]: 8x8 transposes of the input rows
-        for (int q = tid; q < 9 * NCC * (KT / 8); q += WG_NTH) {
-            const int kc = q % (KT / 8), c = (q / (KT / 8)) % NCC, rz = q / ((KT / 8) * NCC);
-            const int dys = rz / 3, dzs = rz % 3;
-            int gy = yy + dys - 1;
-            gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
-            const int gz = zz + dzs - 1;
-            uint4 v[8];
-#pragma unroll
-            for (int a = 0; a < 8; ++a) {
-                const int u = kc * 8 + a;
-                v[a] = make_uint4(0, 0, 0, 0);
-                if (gz >= 0 && gz < nz && u < WT + 2) {
-                    int gx = x0 - 1 + u;
-                    if (nx >= WT) gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
-                    else gx = (gx + nx) % nx;
-                    v[a] = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)gz * ny + gy) * nx + gx) * CIN + c * 8));
-                }
-            }
-            uint4 r[8];
-            transpose8(v, r);
-            unsigned char* dst = sbb + (size_t)dys * L::BD_B + (size_t)kc * (N * 16) + (size_t)(dzs * CIN + c * 8) * 16;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) *reinterpret_cast<uint4*>(dst + e * 16) = r[e];
-        }
-        fence_proxy_async();   // plain stores above are read by the tensor cores
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            constexpr uint32_t IDESC = idesc_bf16(128, N);
-            const uint32_t aaddr = smem_u32(sa), baddr = smem_u32(sbb);
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-#pragma unroll
-                for (int k2 = 0; k2 < KT / 16; ++k2) {
-                    const uint64_t da = smem_desc(aaddr + (uint32_t)(2 * k2) * 2048u, 2048u, 128u);
-                    const uint64_t db = smem_desc(baddr + (uint32_t)(d * L::BD_B + (size_t)(2 * k2) * N * 16),
-                                                  (uint32_t)(N * 16), 128u);
-                    umma_bf16(tmem + (uint32_t)(d * N), da, db, IDESC, (i == 0 && k2 == 0) ? 0u : 1u);
-                }
-            umma_commit(mmadone + b);
-        }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sumdone + st);
+            return true;
+        });
     }
-    // every MMA issued has completed once the last commit of each buffer has
-    const int nmine = i;
-    if (tid == 0) {
-        for (int j = nmine - 2 < 0 ? 0 : nmine - 2; j < nmine; ++j)
-            if (!mbar_wait(mmadone + (j & 1), (unsigned)(j >> 1) & 1u)) *abort_flag = 1;
+    __syncthreads();
+    // the accumulators are complete (after an abort: the MMAs issued have
+    // completed, bounded) once the last commit has
+    if (tid == 0 && *last_commit >= 0) {
+        const int jl = *last_commit;
+        if (!mbar_wait_fast(mmadone + jl % WST, (unsigned)(jl / WST) & 1u)) give_up();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     float* const wrow = ws + (size_t)blockIdx.x * ((size_t)COUT * K + COUT);
-    if (*abort_flag) {
-        if (tid == 0) atomicExch(err, 1);
-    } else if (nmine > 0 && warp < 4) {
-        // accumulator lane m = (dx, n); columns (dz, ci) of y tap d
-        const int m = warp * 32 + lane;
-        const int dxs = m / COUT, n = m % COUT;
+    if (!*abort_flag && warp < 4) {
+        // accumulator lane m = (2-dx, n); columns (dz, ci) of y tap d
+        const int dxs = 2 - tid / COUT, n = tid % COUT;
 #pragma unroll
         for (int d = 0; d < 3; ++d)
 #pragma unroll
             for (int c0 = 0; c0 < N; c0 += 16) {
                 float v[16];
                 tmem_ld<16>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(d * N + c0), v);
-                if (dxs < 3) {
+                if (dxs >= 0) {
+                    float* const o = wrow + (size_t)n * K + (dxs + 3 * d + 9 * (c0 / CIN)) * CIN + c0 % CIN;
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        const int col = c0 + e, dzs = col / CIN, ci = col % CIN;
-                        wrow[(size_t)n * K + (dxs + 3 * d + 9 * dzs) * CIN + ci] = v[e];
-                    }
+                    for (int e = 0; e < 16; ++e) o[e] = v[e];
                 }
             }
-    } else if (nmine == 0 && warp < 4) {
-        // a CTA without segments contributes zeros
-        for (int q = tid; q < COUT * K; q += 128) wrow[q] = 0.f;
     }
     // bias gradient: this thread's 8 channel sums, added up over the threads
     // that hold the same channels, in thread order
+    if (tid < WG_SUM)
 #pragma unroll
-    for (int e = 0; e < 8; ++e) red[tid * 8 + e] = dbacc[e];
+        for (int e = 0; e < 8; ++e) red[tid * 8 + e] = dbacc[e];
     __syncthreads();
     if (tid < COUT) {
-        const int nc = tid / 8, e = tid % 8;
         float sacc = 0.f;
-        for (int t2 = nc; t2 < WG_NTH; t2 += NNC) sacc += red[t2 * 8 + e];
+        for (int t2 = tid / 8; t2 < WG_SUM; t2 += NCY) sacc += red[t2 * 8 + tid % 8];
         wrow[(size_t)COUT * K + tid] = sacc;
     }
     tc_fence_before();
@@ -860,8 +907,17 @@ __global__ void k_wgrad_reduce(const float* __restrict__ ws, int rows, int nw, i
     const int stride = nw + nb;
     const bool bad = *err != 0;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < stride; q += gridDim.x * blockDim.x) {
+        // in row order, 32 loads in flight
         float acc = 0.f;
-        for (int r = 0; r < rows; ++r) acc += ws[(size_t)r * stride + q];
+        int r = 0;
+        for (; r + 32 <= rows; r += 32) {
+            float v[32];
+#pragma unroll
+            for (int t = 0; t < 32; ++t) v[t] = ws[(size_t)(r + t) * stride + q];
+#pragma unroll
+            for (int t = 0; t < 32; ++t) acc += v[t];
+        }
+        for (; r < rows; ++r) acc += ws[(size_t)r * stride + q];
         if (bad) acc = __int_as_float(0x7fc00000);
         if (q < nw) dw[q] += acc;
         else if (db) db[q - nw] += acc;
@@ -963,15 +1019,30 @@ cudaError_t launch_wgrad_tc_t(const void* x, const void* dy, float* dw, float* d
     if (e != cudaSuccess) return e;
     int* err = reinterpret_cast<int*>(static_cast<char*>(buf) + (size_t)grid * stride * sizeof(float));
     e = cudaMemsetAsync(err, 0, sizeof(int), st);
+    // rows of x segments of 64 by TMA: (channel, x, y, z) boxes of 64 voxels
+    CUtensorMap xm, ym;
+    std::memset(&xm, 0, sizeof(xm));
+    std::memset(&ym, 0, sizeof(ym));
+    const int use_tma = nx % WT == 0 ? 1 : 0;
+    if (use_tma && e == cudaSuccess) {
+        for (int o = 0; o < 2 && e == cudaSuccess; ++o) {
+            const cuuint64_t c = o ? COUT : CIN;
+            const cuuint64_t dims[4] = {c, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
+            const cuuint64_t strides[3] = {c * 2, (cuuint64_t)nx * c * 2, (cuuint64_t)nx * ny * c * 2};
+            const cuuint32_t box[4] = {(cuuint32_t)c, (cuuint32_t)WT, 1, 1};
+            e = encode_bf16(o ? &ym : &xm, 4, const_cast<void*>(o ? dy : x), dims, strides, box,
+                            c == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+        }
+    }
     if (e == cudaSuccess) {
         k_conv3d_wgrad_tc<CIN, COUT><<<grid, WG_NTH, L::BYTES, st>>>(
-            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), static_cast<float*>(buf),
+            xm, ym, use_tma, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), static_cast<float*>(buf),
             nx, ny, nz, err);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
         const int nw = COUT * 27 * CIN;
-        k_wgrad_reduce<<<(int)((stride + 255) / 256), 256, 0, st>>>(static_cast<const float*>(buf), grid, nw, COUT,
+        k_wgrad_reduce<<<(int)((stride + 63) / 64), 64, 0, st>>>(static_cast<const float*>(buf), grid, nw, COUT,
                                                                     dw, db, err);
         e = cudaGetLastError();
     }

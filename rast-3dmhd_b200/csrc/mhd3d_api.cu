@@ -14,6 +14,7 @@
 
 #include "../../include/mhd3d.h"
 #include "mhd3d_dev.cuh"
+#include "finalize.cuh"
 #include "ring.cuh"
 #include "smem_attr.cuh"
 
@@ -51,6 +52,7 @@ struct Handle {
     Scalars s{};
     int ntx = 0, nchunks = 0;
     bool dt_valid = false;
+    bool need_reset = true;    // the device's stop flag or accumulators may be set: k_reset before the next step
     unsigned long long w4key = ~0ull;   // key of min over cells of W4 (MHD), else ~0
     // FP32 form: the buffers above hold floats; background profiles
     bool f32 = false;
@@ -357,15 +359,13 @@ __global__ void k_reset(Control* ctl, Accum* acc, int clear_stop, unsigned long 
     acc->wmin[3] = w4key;
     acc->umax = 0ull;
     acc->bad = 0u;
+    acc->done = 0u;
     if (clear_stop) {
         ctl->stop = 0;
         ctl->status = 0;
     }
 }
 
-// End of a step (advance=1: NIT, TIMC, TIMT of STEP 3dmhdsub.f:1171-1173 and
-// the driver's DT check 3dmhd.f:924) and DT/UMACH of the next step from the
-// CFL accumulators (DT=SF*MIN(...), 3dmhdsub.f:866-873; UMACH=SQRT(...), 761).
 // ---- learned closure (no counterpart in the reference) ----------------------
 // Reads of a handle's state as full FP64 values, for either precision.
 struct UView {
@@ -862,38 +862,6 @@ __global__ void k_trip_count(int* flag)
 }
 
 
-__device__ void finalize_one(Control* ctl, Accum* acc, double sf, double dtmin, int lmag, int advance,
-                             unsigned long long w4key)
-{
-    if (advance) {
-        if (ctl->stop) return;
-        ctl->timc = ctl->timc + ctl->dt;
-        ctl->timt = ctl->timi + ctl->timc;
-        ctl->nit += 1;
-        ctl->last_dt = ctl->dt;
-        ctl->last_umach = ctl->umach;
-        if (!(ctl->dt >= dtmin)) {
-            ctl->stop = 1;
-            ctl->status = isfinite(ctl->dt) ? MHD3D_ERR_DT_SMALL : MHD3D_ERR_NONFINITE;
-        }
-    }
-    double w = of_key(acc->wmin[0]);
-    const double w2 = of_key(acc->wmin[1]), w3 = of_key(acc->wmin[2]), w4 = of_key(acc->wmin[3]);
-    w = w2 < w ? w2 : w;
-    w = w3 < w ? w3 : w;
-    if (lmag) w = w4 < w ? w4 : w;
-    ctl->dt = sf * w;
-    ctl->umach = sqrt(of_key(acc->umax));
-    if (acc->bad && !ctl->stop) {
-        ctl->stop = 1;
-        ctl->status = MHD3D_ERR_NONFINITE;
-    }
-    for (int i = 0; i < 3; ++i) acc->wmin[i] = ~0ull;
-    acc->wmin[3] = w4key;
-    acc->umax = 0ull;
-    acc->bad = 0u;
-}
-
 __global__ void k_finalize(Control* ctl, Accum* acc, double sf, double dtmin, int lmag, int advance,
                            unsigned long long w4key)
 {
@@ -944,6 +912,7 @@ StageArgs make_args(Handle* h)
     a.zpitch = h->zpitch;
     a.ntx = h->ntx;
     a.nchunks = h->nchunks;
+    a.w4key = h->w4key;
     a.wait_first = h->wait_first;
     return a;
 }
@@ -985,6 +954,7 @@ StageArgs32 make_args32(Handle* h)
     a.zpitch = h->zpitch;
     a.ntx = h->ntx;
     a.nchunks = h->nchunks;
+    a.w4key = h->w4key;
     return a;
 }
 
@@ -1638,6 +1608,7 @@ int initial_dt(Handle* h)
     k_finalize<<<1, 1, 0, h->st>>>(h->ctl, h->acc, h->s.sf, h->s.dtmin, h->p.lmag, 0, h->w4key);
     CK(cudaGetLastError());
     h->dt_valid = true;
+    h->need_reset = false;
     return MHD3D_OK;
 }
 
@@ -1661,15 +1632,16 @@ int step_async(Handle* h, int n)
 {
     CK(cudaSetDevice(h->dev));
     if (n < 0) return MHD3D_ERR_ARG;
-    // a call that starts from a synced state clears the stop flag; DT of the
-    // current state comes from the last stage-3 reduction, or from a fresh
-    // CFL pass after the state changed
+    // a call that starts from a synced state clears the stop flag, where the
+    // last sync saw it; DT of the current state comes from the last stage-3
+    // reduction, or from a fresh CFL pass after the state changed
     if (!h->dt_valid) {
         int st = initial_dt(h);
         if (st) return st;
-    } else if (h->pending == 0) {
+    } else if (h->pending == 0 && h->need_reset) {
         k_reset<<<1, 1, 0, h->st>>>(h->ctl, h->acc, 1, h->w4key);
         CK(cudaGetLastError());
+        h->need_reset = false;
     }
     int cur = h->cur_base ^ (h->pending & 1);
     for (int s = 0; s < n; ++s) {
@@ -1687,6 +1659,7 @@ int step_async(Handle* h, int n)
                 a.map_u = h->map_u[cur];
                 a.u_in = reinterpret_cast<const float*>(h->ubuf[cur]);
                 a.u_out = reinterpret_cast<float*>(h->ubuf[cur ^ 1]);
+                a.end_step = 1;
                 CK(f32::launch_stage(stg, a, h->st));
             } else {
                 StageArgs a = make_args(h);
@@ -1694,6 +1667,7 @@ int step_async(Handle* h, int n)
                 a.map_o = h->map_o[cur ^ 1];
                 a.u_in = h->ubuf[cur];
                 a.u_out = h->ubuf[cur ^ 1];
+                a.end_step = 1;
                 CK(launch_stage(h, stg, a));
             }
             if (h->prof) {
@@ -1702,9 +1676,7 @@ int step_async(Handle* h, int n)
             }
             cur ^= 1;
         }
-        k_finalize<<<1, 1, 0, h->st>>>(h->ctl, h->acc, h->s.sf, h->s.dtmin, h->p.lmag, 1, h->w4key);
-        CK(cudaGetLastError());
-        h->pending += 1;
+        h->pending += 1;   // stage 3 ended the step (step_end)
     }
     h->cur = cur;
     return MHD3D_OK;
@@ -1716,6 +1688,7 @@ int sync(Handle* h, double* dt, double* timc, double* timt, double* umach, int32
     Control c{};
     CK(cudaMemcpyAsync(&c, h->ctl, sizeof(Control), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
+    if (c.stop) h->need_reset = true;
     // steps after a stop returned at once: the state is where the last completed step left it
     const int ran = c.nit - h->nit_base;
     h->cur = h->cur_base ^ (ran & 1);
@@ -2070,9 +2043,10 @@ int ens_step(Ensemble* e, int nsteps)
         if (!h->dt_valid) {
             int st = initial_dt(h);
             if (st) return st;
-        } else if (h->pending == 0) {
+        } else if (h->pending == 0 && h->need_reset) {
             k_reset<<<1, 1, 0, h->st>>>(h->ctl, h->acc, 1, h->w4key);
             CK(cudaGetLastError());
+            h->need_reset = false;
         }
         const int cur = h->cur_base ^ (h->pending & 1);
         cur0[i] = cur;
@@ -2166,6 +2140,7 @@ int ens_tune(Ensemble* e, int steps, int32_t* zlen_out, int32_t* ctas_out, doubl
             h->nit_base = saved_nit[i];
             h->pending = 0;
             h->dt_valid = saved_valid[i];
+            h->need_reset = true;
         }
         CK(cudaStreamSynchronize(e->st));
         return MHD3D_OK;
@@ -2364,6 +2339,7 @@ int mhd3d_cfl(void* handle, double* dt, double* umach)
     Control c{};
     CK(cudaMemcpyAsync(&c, h->ctl, sizeof(Control), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
+    if (c.stop) h->need_reset = true;
     if (dt) *dt = c.dt;
     if (umach) *umach = c.umach;
     return c.stop ? c.status : MHD3D_OK;

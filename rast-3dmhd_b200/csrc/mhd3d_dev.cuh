@@ -88,7 +88,7 @@ struct Accum {
     unsigned long long wmin[4];
     unsigned long long umax;
     unsigned int bad;
-    unsigned int pad;
+    unsigned int done;   // stage-3 CTAs that have added their parts
 };
 
 struct Metrics {
@@ -141,6 +141,8 @@ struct StageArgs {
     int upitch, zpitch;
     int ntx;                // tiles along x
     int nchunks;            // z chunks (chunk_start)
+    int end_step;           // the last CTA of stage 3 ends the step (finalize.cuh)
+    unsigned long long w4key;
     long long wait_first;   // poll limit of a CTA's first ring wait (WAIT_LIMIT; lowered only by tests)
 };
 
@@ -222,6 +224,8 @@ struct StageArgs32 {
     size_t uf, uz, zf, zz;
     int upitch, zpitch;
     int ntx, nchunks;
+    int end_step;             // as StageArgs
+    unsigned long long w4key;
 };
 
 // first plane of z chunk c of n: chunks differ by one plane at most

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     const bool active = gi < npx && gj < npy;
     const int lx = tx + BXO, ly = ty + 1;
 
+    grid_wait();   // what follows reads what the kernels before wrote
     const double DT = ctl->dt;
     const double cu = STAGE == 1 ? s.gam1 * DT : STAGE == 2 ? s.gam2 * DT : s.gam3 * DT;   // COEF for U
     const double cz = STAGE == 1 ? s.zeta1 * DT : s.zeta2 * DT;                            // COEF for Z
@@ -565,6 +566,9 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
         }
         return;
     }
-    if (STAGE == 3) cfl_commit_acc(a.acc, red, cfa);
+    if (STAGE == 3) {
+        cfl_commit_acc(a.acc, red, cfa);
+        if (tid == 0) step_end(a);
+    }
 }
 

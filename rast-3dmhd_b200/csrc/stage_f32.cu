@@ -29,6 +29,7 @@
 #define MHD3D_NS f32
 #define MHD3D_FAST_BODY 1
 #include "cfl_cell.cuh"
+#include "finalize.cuh"
 
 namespace mhd3d {
 namespace f32 {
@@ -596,6 +597,7 @@ __device__ __forceinline__ void stage32_item(const StageArgs32& a, const int til
         }
     } else if (STAGE == 3) {
         cfl32_commit(a.acc, red, cfa);
+        if (tid == 0) step_end(a);
     }
     __syncthreads();
     if (tid == 0)
@@ -607,6 +609,7 @@ __global__ void __launch_bounds__(NT32, MHD3D_MINB32) k_stage32(const __grid_con
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* const sb = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    grid_wait();   // what follows reads what the kernels before wrote
     stage32_item<MAG, ROT, STAGE>(a, blockIdx.x, blockIdx.y, sb);
 }
 
@@ -721,8 +724,7 @@ static cudaError_t launch_stage_t(int stage, const StageArgs32& a, cudaStream_t 
         static std::atomic<unsigned long long> attr_set{0};                                                \
         cudaError_t ae = smem_attr_once(attr_set, reinterpret_cast<const void*>(k_stage32<MAG, ROT, S>), smem); \
         if (ae != cudaSuccess) return ae;                                                                  \
-        k_stage32<MAG, ROT, S><<<grid, NT32, smem, st>>>(a);                                              \
-        break;                                                                                             \
+        return launch_chained(k_stage32<MAG, ROT, S>, grid, NT32, smem, st, a);                           \
     }
         L_(0) L_(1) L_(2) L_(3)
 #undef L_

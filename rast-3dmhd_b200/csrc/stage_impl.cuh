@@ -26,6 +26,7 @@
 #include "mhd3d_dev.cuh"
 #include "smem_attr.cuh"
 #include "cfl_cell.cuh"
+#include "finalize.cuh"
 #include "ring.cuh"
 #if MHD3D_FAST_BODY
 #include "march.cuh"
@@ -198,8 +199,7 @@ static cudaError_t launch_stage_t(int stage, const StageArgs& a, cudaStream_t st
         static std::atomic<unsigned long long> attr_set{0};                                                \
         cudaError_t ae = smem_attr_once(attr_set, reinterpret_cast<const void*>(k_stage<MAG, ROT, S>), smem); \
         if (ae != cudaSuccess) return ae;                                                                  \
-        k_stage<MAG, ROT, S><<<grid, NT, smem, st>>>(a);                                                  \
-        break;                                                                                             \
+        return launch_chained(k_stage<MAG, ROT, S>, grid, NT, smem, st, a);                                      \
     }
         L_(0) L_(1) L_(2) L_(3)
 #undef L_

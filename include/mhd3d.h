@@ -303,10 +303,8 @@ int mhd3d_ensemble_set_stream(void* ens, void* stream);
  * arrays are device pointers; activations are channels-last BF16
  * [nz][ny][nx][C] (periodic in x and y, zero outside in z), weights BF16
  * [cout][27*cin] with k = tap*cin + ci, tap = (dx+1) + 3*(dy+1) + 9*(dz+1).
- * Any nx >= 1 (x segments of 128 voxels; a segment that runs past the row's
- * end, or a row shorter than 128, wraps periodically and stores only its own
- * voxels; nx a multiple of 128 takes the TMA loader); every array is 16-byte
- * aligned.
+ * Any nx >= 1 (x segments of 128 voxels, the last one shorter); every array
+ * is 16-byte aligned.
  * Supported (cin, cout): (16,32), (32,32),
  * (32,16).  Work is enqueued on stream; err (device int) is set non-zero if
  * a bounded wait of the tensor-core pipeline gave up.

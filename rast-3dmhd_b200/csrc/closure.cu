@@ -12,18 +12,15 @@
 //    M=128, K=16 per instruction) issued by one thread.  Input rows (130 x
 //    3 z planes) sit in a shared-memory ring, so the A operand of tap
 //    (dx, dz) is one descriptor moved by whole voxel rows: with 32 input
-//    channels and x a multiple of 128, 64-byte voxel rows in the copy
-//    engine's 64-byte swizzle (one TMA box per plane); otherwise
-//    [8-channel chunk][voxel] 16-byte rows, the canonical K-major no-swizzle
-//    layout with 8-row groups 128 bytes apart.  Any nx: a tile that runs past
-//    the row's end reads the row again from its start (periodic), and only
-//    its first nx - x0 outputs are stored (for nx < 128 the tile holds the
-//    row's period more than once).  One MMA serves three output rows (N = 3*COUT,
+//    channels, 64-byte voxel rows in the copy engine's 64-byte swizzle (one
+//    TMA box per plane); with 16, [8-channel chunk][voxel] 16-byte rows, the
+//    canonical K-major no-swizzle layout with 8-row groups 128 bytes apart.
+//    Any nx: the boxes of a row's last segment end with the row, and only its
+//    own outputs are stored.  One MMA serves three output rows (N = 3*COUT,
 //    the y taps stacked in the B operand), see k_conv3d.  Warp roles: a
-//    loader (TMA boxes, or cp.async when nx is not a multiple of 128), one
-//    MMA thread and four epilogue warps, handing off through mbarriers.  The
-//    epilogue adds the bias, applies ReLU or the ReLU mask of the layer
-//    below, and writes BF16 (and FP32) outputs.
+//    loader, one MMA thread and four epilogue warps, handing off through
+//    mbarriers.  The epilogue adds the bias, applies ReLU or the ReLU mask of
+//    the layer below, and writes BF16 (and FP32) outputs.
 //  - k_conv3d_wgrad_tc: dW[n][tap*CIN+ci] = sum over voxels of dY[v][n] *
 //    X[v+tap][ci] on tcgen05 as well, with K running over voxels: per x
 //    segment a dY row read at the three x shifts forms A and the input rows
@@ -46,11 +43,9 @@
 namespace mhd3d {
 namespace clo {
 
-constexpr int NLW = 4;             // loader warps of a convolution CTA
-constexpr int CT = 32 * (4 + NLW + 1);   // threads: 4 epilogue warps (TMEM lanes 0..127), loaders, MMA
+constexpr int CT = 32 * (4 + 1 + 1);     // threads: 4 epilogue warps (TMEM lanes 0..127), loader, MMA
 constexpr int RING = 4;            // input rows held in the ring: the loaders run up to three steps ahead
 constexpr int MT = 128;            // output voxels per tile: one 128-point x segment
-constexpr int BX = MT + 2;         // input block: x with halo
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -128,45 +123,22 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float (&v)[32])
 // voxels start on a 128-byte (512-byte) boundary, a TMA destination; step s
 // of a CTA keeps its input row in slot s % RING.
 constexpr int XR0 = 7;
-constexpr int BXP = 144;              // XR0 + BX rounded up to 8 rows
+constexpr int BXP = 144;              // XR0 + MT + 2 rounded up to 8 rows
 constexpr int RSEG = RING * 3 * BXP;  // voxel rows of one chunk of the ring
-template <int CIN, int NTH>
-__device__ __forceinline__ void load_row_async(unsigned char* ring, const __nv_bfloat16* __restrict__ x, int x0,
-                                               int yr, int z, int nx, int ny, int nz, int tix, int slot)
-{
-    constexpr int NC = CIN / 8;
-    int gy = yr % ny;
-    gy = gy < 0 ? gy + ny : gy;
-    const uint32_t sbase = smem_u32(ring);
-    for (int q = tix; q < 3 * BX * NC; q += NTH) {
-        const int c = q / (3 * BX), r = q % (3 * BX);
-        const int zi = r / BX, xi = r % BX;
-        int gx = x0 - 1 + xi;
-        if (nx >= MT) gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
-        else gx = (gx + nx) % nx;   // a 128-point tile spans 128/nx periods
-        int gz = z - 1 + zi;
-        const uint32_t nbytes = (gz >= 0 && gz < nz) ? 16u : 0u;
-        gz = gz < 0 ? 0 : (gz >= nz ? nz - 1 : gz);
-        const __nv_bfloat16* src = x + (((size_t)gz * ny + gy) * nx + gx) * CIN + c * 8;
-        const uint32_t dst = sbase + (uint32_t)((c * RSEG + (slot * 3 + zi) * BXP + XR0 + xi) * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(nbytes) : "memory");
-    }
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// The input row of a step by TMA (x segments of 128 voxels, nx a multiple of
-// 128): one 5-D box (8 channels, 1 chunk, 128 x, 1 y, 1 z) per chunk and z
+// The input row of a step by TMA (w <= 128 voxels from x0, the width of map's
+// boxes): one 5-D box (8 channels, 1 chunk, w x, 1 y, 1 z) per chunk and z
 // plane into the ring's interior rows, zeros outside z (out-of-range box);
-// the two periodic x halo voxels by cp.async from the calling warp.  The
+// the two periodic x halo voxels by cp.async from the calling warp.  What a
+// short row leaves behind its halo feeds only outputs that are not stored.  The
 // TMA bytes complete on bar (after the caller's expect_tx); each lane's
 // copies are signalled by the caller's cp.async.mbarrier.arrive.
 template <int CIN>
 __device__ __forceinline__ void load_row_tma(unsigned char* ring, const CUtensorMap* map, unsigned long long* bar,
-                                             const __nv_bfloat16* __restrict__ x, int x0, int yr, int z, int nx,
-                                             int ny, int nz, int lane, int slot)
+                                             const __nv_bfloat16* __restrict__ x, int x0, int w, int yr, int z,
+                                             int nx, int ny, int nz, int lane, int slot)
 {
     constexpr int NC = CIN / 8;
     int gy = yr % ny;
@@ -186,7 +158,7 @@ __device__ __forceinline__ void load_row_tma(unsigned char* ring, const CUtensor
     }
     for (int q = lane; q < 2 * NC * 3; q += 32) {
         const int side = q & 1, c = (q >> 1) % NC, zi = (q >> 1) / NC;
-        const int xi = side ? BX - 1 : 0;
+        const int xi = side ? w + 1 : 0;
         int gx = x0 - 1 + xi;
         gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
         int gz = z - 1 + zi;
@@ -204,12 +176,13 @@ __device__ __forceinline__ void load_row_tma(unsigned char* ring, const CUtensor
 // chunk j (channels 8j..8j+7) of row R sits at chunk position j ^ ((R >> 1) & 3)
 // -- the copy engine's SWIZZLE_64B pattern (address bits 4-5 XOR bits 7-8,
 // planes 512-byte aligned), which SWIZZLE_64B matrix descriptors read back.
-// One 4-D box (32 channels, 128 x, 1 y, 1 z) per plane lands the interior at
+// One 4-D box (32 channels, w x, 1 y, 1 z) per plane lands the interior at
 // row XR0+1; the two periodic halo voxels come by cp.async, placed by the
 // same rule.
 __device__ __forceinline__ void load_row_tma_sw64(unsigned char* ring, const CUtensorMap* map,
                                                   unsigned long long* bar, const __nv_bfloat16* __restrict__ x,
-                                                  int x0, int yr, int z, int nx, int ny, int nz, int lane, int slot)
+                                                  int x0, int w, int yr, int z, int nx, int ny, int nz, int lane,
+                                                  int slot)
 {
     constexpr int CIN = 32;
     int gy = yr % ny;
@@ -228,7 +201,7 @@ __device__ __forceinline__ void load_row_tma_sw64(unsigned char* ring, const CUt
     }
     if (lane < 24) {
         const int side = lane & 1, j = (lane >> 1) & 3, zi = lane >> 3;
-        const int xi = side ? BX - 1 : 0;
+        const int xi = side ? w + 1 : 0;
         int gx = x0 - 1 + xi;
         gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
         int gz = z - 1 + zi;
@@ -349,23 +322,28 @@ struct ConvLay {
 // stores.  The first MMA of a run starts all three slots from zero.
 //
 // Warp roles, pipelined over the CTA's steps s (ready and mmadone by s & 3):
-//   loaders: the step's input row (three z planes, periodic in x and y,
-//     zeros outside z) into ring slot s % RING.  With use_tma (nx a multiple
-//     of 128) warp 4 alone: one TMA box per z plane of 32 channels x 128
-//     voxels in 64-byte swizzled rows (CIN = 32), or of 8 channels x 128
-//     voxels per chunk and plane (CIN = 16), complete_tx on ready(s), and
-//     the two x-halo voxels by cp.async; otherwise warps 4..4+NLW-1 by
-//     cp.async.  Each loader thread's
-//     copies arrive on ready(s) as they land (cp.async.mbarrier.arrive), and a
-//     slot is reused once the MMAs of step s - RING have completed (mmadone).
-//   warp 4+NLW, lane 0 (MMA): waits ready(s) and the release of step s-1's
+//   loader (warp 4): the step's input row (three z planes, periodic in x and y,
+//     zeros outside z) into ring slot s % RING: one TMA box per z plane of 32
+//     channels x 128 voxels (fewer at the row's end) in 64-byte swizzled rows
+//     (CIN = 32), or of 8 channels x 128 voxels per chunk and plane (CIN = 16),
+//     complete_tx on ready(s), and the two x-halo voxels by cp.async, which
+//     arrive on ready(s) as they land (cp.async.mbarrier.arrive); a slot is
+//     reused once the MMAs of step s - RING have completed (mmadone).
+//   warp 5, lane 0 (MMA): waits ready(s) and the release of step s-1's
 //     finished slot (accempty), issues the step's MMAs, commits to accfull
 //     and to mmadone(s).
 //   warps 0-3 (epilogue): wait accfull(s), read and zero the finished slot
 //     (TMEM lanes 32*warp..), release it (accempty) and store while the next
 //     step's MMAs run.
+//
+// A row's last segment has boxes of its own width rather than voxels copied
+// one by one with the wrap computed for each: us at nx x 128 x 64, 16->32,
+// 32->32, 32->16, before and now: nx = 55: 105, 169, 157 / 63, 81, 71;
+// 250 (one full segment, one of 122): 154, 234, 211 / 112, 142, 124; 128
+// (full segments only): 65, 83, 72.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtensorMap xmap, int use_tma,
+__global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtensorMap xmap,
+                                                  const __grid_constant__ CUtensorMap xtail,
                                                   const __nv_bfloat16* __restrict__ x,
                                                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
                                                   const __nv_bfloat16* __restrict__ mask, int relu,
@@ -424,9 +402,8 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
     }
     if (tid == 0) {
         for (int b = 0; b < 4; ++b) {
-            // TMA: the expect_tx arrival and one completion arrival per lane of
-            // the loader warp; cp.async only: one per loader thread
-            mbar_init(ready + b, use_tma ? 1 + 32 : 32 * NLW);
+            // the expect_tx arrival and one completion arrival per lane of the loader warp
+            mbar_init(ready + b, 1 + 32);
             mbar_init(mmadone + b, 1);
         }
         mbar_init(accfull, 1);
@@ -452,7 +429,7 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
         atomicExch(err, 1);
     };
 
-    if (use_tma && warp == 4) {
+    if (warp == 4) {
         // one warp: the TMA boxes of the step's row and its two halo voxels
         for_steps(t_begin, t_end, ny, nz, [&](int s, int x0, int zz, int r, bool, bool) {
             if (*abort_flag) return false;
@@ -462,32 +439,16 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
                 return false;
             }
             unsigned long long* const bar = ready + (s & 3);
-            if (lane == 0) mbar_expect_tx(bar, (unsigned)(CIN / 8 * 3 * MT * 16));
-            if constexpr (CIN == 32) load_row_tma_sw64(sx, &xmap, bar, x, x0, r, zz, nx, ny, nz, lane, s % RING);
-            else load_row_tma<CIN>(sx, &xmap, bar, x, x0, r, zz, nx, ny, nz, lane, s % RING);
+            const int w = nx - x0 < MT ? nx - x0 : MT;
+            const CUtensorMap* const map = w < MT ? &xtail : &xmap;
+            if (lane == 0) mbar_expect_tx(bar, (unsigned)(CIN / 8 * 3 * w * 16));
+            if constexpr (CIN == 32) load_row_tma_sw64(sx, map, bar, x, x0, w, r, zz, nx, ny, nz, lane, s % RING);
+            else load_row_tma<CIN>(sx, map, bar, x, x0, w, r, zz, nx, ny, nz, lane, s % RING);
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
             return true;
         });
         cp_async_wait<0>();
-    } else if (!use_tma && warp >= 4 && warp < 4 + NLW) {
-        // each loader thread's copies of step s arrive on ready(s) when they
-        // land, so the loaders run ahead as far as the ring allows
-        const int tix = tid - 128;
-        for_steps(t_begin, t_end, ny, nz, [&](int s, int x0, int zz, int r, bool, bool) {
-            if (*abort_flag) return false;
-            // slot s % RING was last read by step s - RING
-            const int jw = s - RING;
-            if (jw >= 0 && !mbar_wait_fast(mmadone + (jw & 3), (unsigned)(jw >> 2) & 1u)) {
-                give_up();
-                return false;
-            }
-            load_row_async<CIN, 32 * NLW>(sx, x, x0, r, zz, nx, ny, nz, tix, s % RING);
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(ready + (s & 3)))
-                         : "memory");
-            return true;
-        });
-        cp_async_wait<0>();
-    } else if (warp == 4 + NLW) {
+    } else if (warp == 5) {
         if (lane == 0) {
             constexpr uint32_t IDESC = idesc_bf16(MT, L::NW);
             const uint64_t da0 = smem_desc(smem_u32(sx), RSEG * 16, 128);
@@ -512,7 +473,7 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
                 // bytes into the row), 16-byte rows otherwise (the second K
                 // half one chunk of the ring further)
                 constexpr int NM = 9 * CIN / 16, KH = CIN / 16;
-                const bool swz = CIN == 32 && use_tma;
+                constexpr bool swz = CIN == 32;
                 const uint64_t dab = swz ? da0s : da0;
                 const uint32_t a0 = (uint32_t)dab + (swz ? as * 4 : as);
                 const uint32_t b0 = (uint32_t)db0 + st * (COUT / 8) * (KB / 8) * 8;
@@ -535,7 +496,7 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
             });
         }
         __syncwarp();
-    } else if (warp < 4) {   // loader warps without work (TMA rows) take no role
+    } else {
         for_steps(t_begin, t_end, ny, nz, [&](int s, int x0, int zz, int r, bool, bool emit) {
             if (*abort_flag) return false;
             if (!mbar_wait_fast(accfull, (unsigned)s & 1u)) {
@@ -612,12 +573,12 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
 // Channels-last rows are MN-major operands as they lie in memory: a voxel is
 // one row of K, its channels one row of M or N (64- or 32-byte rows in the
 // swizzle of that width, which the matrix descriptors read back), so TMA boxes
-// of 64 voxels (x a multiple of 64; the two halo voxels, and any other row, by
-// cp.async) fill both operands and nothing is transposed.  The x taps are blocks of one
-// staged dY row that start a voxel apart (block j holds dx = 2-j; the leading
-// offset of A is one voxel; blocks beyond the third are unused lanes), the z
-// taps the three planes of an input row.  The loader warps run up to WST
-// segments ahead of the MMA thread.  The three accumulators (3*3*CIN columns)
+// (and cp.async for the two halo voxels) fill both operands and nothing is
+// transposed.  The x taps are blocks of one staged dY row that start a voxel
+// apart (block j holds dx = 2-j; the leading offset of A is one voxel; blocks
+// beyond the third are unused lanes), the z taps the three planes of an input
+// row.  A row's last segment has boxes of its own width and only the K steps
+// that its voxels reach.  The loader warp runs up to WST segments ahead of the MMA thread.  The three accumulators (3*3*CIN columns)
 // stay in TMEM over all of a CTA's segments (a fixed set, in a fixed order);
 // each CTA writes its partial sums to a workspace row and a second kernel adds
 // the rows to dW in CTA order, so the result does not depend on timing.
@@ -625,12 +586,12 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
 // Bound by L2 reads (42 KB a segment for 32 input channels) and the hand-offs
 // of three stages; 128x128x64, us: 16->32 117, 32->32 143, 32->16 129.  The
 // form that transposed both operands through registers took 463, 657 and 605,
-// this one with every row by cp.async 151, 241 and 231.  Marching along y with
+// this one with every voxel by cp.async 151, 241 and 231.  Marching along y with
 // 128-voxel segments and the roles of the operands exchanged took 137, 146 and
 // 114, but sums in another order; this one's bits are those of the first form.
 constexpr int WT = 64;               // voxels of an x segment
 constexpr int KT = 80;               // K of a segment: WT + 2 halo voxels, padded to 16
-constexpr int WG_LD = 8;             // loader warps
+constexpr int WG_LD = 1;             // loader warp
 constexpr int WG_SUM = 256;          // threads that sum dY (the first four warps are the epilogue)
 constexpr int WG_NTH = WG_SUM + 32 * (WG_LD + 1);
 // Rows of the staged operands: voxel x0 of an input row or of dY sits at row 8,
@@ -684,7 +645,8 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool o
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_constant__ CUtensorMap xmap,
-                                                               const __grid_constant__ CUtensorMap ymap, int use_tma,
+                                                               const __grid_constant__ CUtensorMap xtail,
+                                                               const __grid_constant__ CUtensorMap ymap,
                                                                const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ dy,
                                                                float* __restrict__ ws, int nx, int ny, int nz,
@@ -715,7 +677,7 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_cons
     }
     if (tid == 0) {
         for (int b = 0; b < WST; ++b) {
-            mbar_init(ready + b, use_tma ? 1 + 32 : 32 * WG_LD);
+            mbar_init(ready + b, 1 + 32);
             mbar_init(mmadone + b, 1);
             mbar_init(sumdone + b, WG_SUM / 32);
         }
@@ -750,20 +712,26 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_cons
         return false;
     };
 
+    // K steps of a segment of w voxels: u = 0..w+1 can meet a dY of its own
+    auto ksteps = [](int w) { return (w + 2 + 15) / 16; };
+
     float dbacc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // dY sums of this thread's 8 channels
-    if (use_tma && warp == WG_SUM / 32) {
-        // one warp: ten TMA boxes and the input rows' halo voxels
+    if (warp == WG_SUM / 32) {
+        // one warp: ten TMA boxes (dY zeros beyond the row's end) and the input
+        // rows' halo voxels; what a short row leaves behind its halo meets zeros
         segments([&](int i, int t, int st, unsigned ph) {
             if (i >= WST && (!mbar_wait_fast(mmadone + st, ph ^ 1u) || !mbar_wait_fast(sumdone + st, ph ^ 1u)))
                 return give_up();
             const int x0 = (t % nseg) * WT, yy = (t / nseg) % ny, zz = t / (nseg * ny);
             const uint32_t sx = sa + (uint32_t)(st * L::STAGE_B);
+            const int w = nx - x0 < WT ? nx - x0 : WT;   // the segment's own voxels
+            const CUtensorMap* const map = w < WT ? &xtail : &xmap;
             if (lane == 0) {
-                mbar_expect_tx(ready + st, (unsigned)(9 * WT * L::XB + WT * L::YB));
+                mbar_expect_tx(ready + st, (unsigned)(9 * w * L::XB + WT * L::YB));
                 for (int rz = 0; rz < 9; ++rz) {
                     int gy = yy + rz / 3 - 1;
                     gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
-                    tma_load4(sb + (size_t)st * L::STAGE_B + rz * L::X_ROW + 8 * L::XB, &xmap, ready + st, 0, x0, gy,
+                    tma_load4(sb + (size_t)st * L::STAGE_B + rz * L::X_ROW + 8 * L::XB, map, ready + st, 0, x0, gy,
                               zz + rz % 3 - 1);   // zeros outside z
                 }
                 tma_load4(sb + (size_t)st * L::STAGE_B + L::Y_OFF + 8 * L::YB, &ymap, ready + st, 0, x0, yy, zz);
@@ -774,44 +742,18 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_cons
                 gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
                 const int gz = zz + rz % 3 - 1;
                 const bool on = gz >= 0 && gz < nz;
-                int gx = side ? x0 + WT : x0 - 1;
+                int gx = side ? x0 + w : x0 - 1;
                 gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
-                cp_async16(sx + (uint32_t)(rz * L::X_ROW) + swz_chunk<L::XB>(side ? 8 + WT : 7, c),
+                cp_async16(sx + (uint32_t)(rz * L::X_ROW) + swz_chunk<L::XB>(side ? 8 + w : 7, c),
                            x + (((size_t)(on ? gz : zz) * ny + gy) * nx + gx) * CIN + c * 8, on);
             }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(ready + st)) : "memory");
-            return true;
-        });
-        cp_async_wait<0>();
-    } else if (!use_tma && tid >= WG_SUM && warp < WG_SUM / 32 + WG_LD) {
-        const int lt = tid - WG_SUM;
-        segments([&](int i, int t, int st, unsigned ph) {
-            // the stage was last read by the segment WST before
-            if (i >= WST && (!mbar_wait_fast(mmadone + st, ph ^ 1u) || !mbar_wait_fast(sumdone + st, ph ^ 1u)))
-                return give_up();
-            const int x0 = (t % nseg) * WT, yy = (t / nseg) % ny, zz = t / (nseg * ny);
-            const uint32_t sx = sa + (uint32_t)(st * L::STAGE_B), sy = sx + L::Y_OFF;
-            const __nv_bfloat16* const drow = dy + (((size_t)zz * ny + yy) * nx + x0) * COUT;
-            const int mlim = nx - x0 < WT ? nx - x0 : WT;   // the segment's own voxels (nx < 64: one period)
-            for (int q = lt; q < WT * NCY; q += 32 * WG_LD) {
-                const int c = q % NCY, j = q / NCY;
-                cp_async16(sy + swz_chunk<L::YB>(j + 8, c), drow + (size_t)(j < mlim ? j : 0) * COUT + c * 8, j < mlim);
-            }
-            // a (row, voxel) pair a step of the loop: its chunks by adjacent threads
-            constexpr int RP = 32 * WG_LD / NCX;   // pairs in flight over the loaders
-            const int c = lt % NCX;
-            for (int q = lt / NCX; q < 9 * (WT + 2); q += RP) {
-                const int rz = q / (WT + 2), u = q % (WT + 2);
-                int gy = yy + rz / 3 - 1;
-                gy = gy < 0 ? gy + ny : (gy >= ny ? gy - ny : gy);
-                const int gz = zz + rz % 3 - 1;
-                const bool on = gz >= 0 && gz < nz;
-                int gx = x0 - 1 + u;
-                if (nx >= WT) gx = gx < 0 ? gx + nx : (gx >= nx ? gx - nx : gx);
-                else gx = (gx + nx) % nx;
-                cp_async16(sx + (uint32_t)(rz * L::X_ROW) + swz_chunk<L::XB>(WXR0 + u, c),
-                           x + (((size_t)(on ? gz : zz) * ny + gy) * nx + gx) * CIN + c * 8, on);
-            }
+            // a short segment: zeros up to the end of its last K step
+            const int nzr = ksteps(w) * 16 - (w + 2);
+            if (w < WT)
+                for (int q = lane; q < 9 * nzr * NCX; q += 32) {
+                    const int c = q % NCX, u = q / NCX % nzr, rz = q / (nzr * NCX);
+                    cp_async16(sx + (uint32_t)(rz * L::X_ROW) + swz_chunk<L::XB>(9 + w + u, c), x, false);
+                }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(ready + st)) : "memory");
             return true;
         });
@@ -819,8 +761,9 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_cons
     } else if (warp == WG_SUM / 32 + WG_LD) {
         if (lane == 0) {
             constexpr uint32_t IDESC = idesc_bf16(128, N) | (1u << 15) | (1u << 16);   // both operands MN-major
-            segments([&](int i, int, int st, unsigned ph) {
+            segments([&](int i, int t, int st, unsigned ph) {
                 if (!mbar_wait_fast(ready + st, ph)) return give_up();
+                const int x0 = (t % nseg) * WT, ks = ksteps(nx - x0 < WT ? nx - x0 : WT);
                 fence_proxy_async();   // rows written by cp.async are read by the tensor cores
                 tc_fence_after();
                 const uint32_t sx = sa + (uint32_t)(st * L::STAGE_B);
@@ -829,10 +772,12 @@ __global__ void __launch_bounds__(WG_NTH, 1) k_conv3d_wgrad_tc(const __grid_cons
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
 #pragma unroll
-                    for (int k2 = 0; k2 < KT / 16; ++k2)
+                    for (int k2 = 0; k2 < KT / 16; ++k2) {
+                        if (k2 >= ks) break;
                         umma_bf16(tmem + (uint32_t)(d * N), da + (uint64_t)(k2 * L::YB),
                                   db + (uint64_t)((d * 3 * L::X_ROW >> 4) + k2 * L::XB), IDESC,
                                   (i == 0 && k2 == 0) ? 0u : 1u);
+                    }
                 umma_commit(mmadone + st);
                 *last_commit = i;
                 return true;
@@ -970,28 +915,31 @@ cudaError_t launch_conv_t(const void* x, const void* w, const float* bias, const
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int ntile = ((nx + MT - 1) / MT) * ny * nz;
     const int grid = ntile < sms ? ntile : sms;
-    // rows of x segments of 128 by TMA: (8 channels, chunk, x, y, z) boxes
-    CUtensorMap map;
-    std::memset(&map, 0, sizeof(map));
-    const int use_tma = nx % MT == 0 ? 1 : 0;
-    if (use_tma && CIN == 32) {
-        // (channel, x, y, z) boxes of 32 channels x 128 voxels, 64-byte swizzled rows
-        const cuuint64_t dims[4] = {(cuuint64_t)CIN, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
-        const cuuint64_t strides[3] = {(cuuint64_t)CIN * 2, (cuuint64_t)nx * CIN * 2, (cuuint64_t)nx * ny * CIN * 2};
-        const cuuint32_t box[4] = {(cuuint32_t)CIN, (cuuint32_t)MT, 1, 1};
-        if (encode_bf16(&map, 4, const_cast<void*>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B) != cudaSuccess)
-            return cudaErrorInvalidValue;
-    } else if (use_tma) {
-        // (8 channels, chunk, x, y, z) boxes, 16-byte rows
-        const cuuint64_t dims[5] = {8, (cuuint64_t)CIN / 8, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
-        const cuuint64_t strides[4] = {16, (cuuint64_t)CIN * 2, (cuuint64_t)nx * CIN * 2,
-                                       (cuuint64_t)nx * ny * CIN * 2};
-        const cuuint32_t box[5] = {8, 1, (cuuint32_t)MT, 1, 1};
-        if (encode_bf16(&map, 5, const_cast<void*>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE) != cudaSuccess)
-            return cudaErrorInvalidValue;
+    // boxes of 128 voxels, and of what the row's last segment holds
+    CUtensorMap maps[2];
+    std::memset(maps, 0, sizeof(maps));
+    for (int o = 0; o < 2; ++o) {
+        const int w = o ? nx % MT : MT;
+        if (!w || (!o && nx < MT)) continue;
+        cudaError_t e;
+        if (CIN == 32) {
+            // (channel, x, y, z) boxes of 32 channels, 64-byte swizzled rows
+            const cuuint64_t dims[4] = {(cuuint64_t)CIN, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
+            const cuuint64_t strides[3] = {(cuuint64_t)CIN * 2, (cuuint64_t)nx * CIN * 2, (cuuint64_t)nx * ny * CIN * 2};
+            const cuuint32_t box[4] = {(cuuint32_t)CIN, (cuuint32_t)w, 1, 1};
+            e = encode_bf16(&maps[o], 4, const_cast<void*>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B);
+        } else {
+            // (8 channels, chunk, x, y, z) boxes, 16-byte rows
+            const cuuint64_t dims[5] = {8, (cuuint64_t)CIN / 8, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
+            const cuuint64_t strides[4] = {16, (cuuint64_t)CIN * 2, (cuuint64_t)nx * CIN * 2,
+                                           (cuuint64_t)nx * ny * CIN * 2};
+            const cuuint32_t box[5] = {8, 1, (cuuint32_t)w, 1, 1};
+            e = encode_bf16(&maps[o], 5, const_cast<void*>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+        }
+        if (e != cudaSuccess) return e;
     }
     k_conv3d<CIN, COUT><<<grid, CT, L::BYTES, st>>>(
-        map, use_tma, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), bias,
+        maps[0], maps[1], static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), bias,
         static_cast<const __nv_bfloat16*>(mask), relu, static_cast<__nv_bfloat16*>(y), yf, nx, ny, nz, err);
     return cudaGetLastError();
 }
@@ -1019,25 +967,23 @@ cudaError_t launch_wgrad_tc_t(const void* x, const void* dy, float* dw, float* d
     if (e != cudaSuccess) return e;
     int* err = reinterpret_cast<int*>(static_cast<char*>(buf) + (size_t)grid * stride * sizeof(float));
     e = cudaMemsetAsync(err, 0, sizeof(int), st);
-    // rows of x segments of 64 by TMA: (channel, x, y, z) boxes of 64 voxels
-    CUtensorMap xm, ym;
-    std::memset(&xm, 0, sizeof(xm));
-    std::memset(&ym, 0, sizeof(ym));
-    const int use_tma = nx % WT == 0 ? 1 : 0;
-    if (use_tma && e == cudaSuccess) {
-        for (int o = 0; o < 2 && e == cudaSuccess; ++o) {
-            const cuuint64_t c = o ? COUT : CIN;
-            const cuuint64_t dims[4] = {c, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
-            const cuuint64_t strides[3] = {c * 2, (cuuint64_t)nx * c * 2, (cuuint64_t)nx * ny * c * 2};
-            const cuuint32_t box[4] = {(cuuint32_t)c, (cuuint32_t)WT, 1, 1};
-            e = encode_bf16(o ? &ym : &xm, 4, const_cast<void*>(o ? dy : x), dims, strides, box,
-                            c == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-        }
+    // (channel, x, y, z) boxes: 64 voxels of x and dy, and of x what the row's last segment holds
+    CUtensorMap maps[3];
+    std::memset(maps, 0, sizeof(maps));
+    for (int o = 0; o < 3 && e == cudaSuccess; ++o) {
+        const int w = o == 1 ? nx % WT : WT;
+        if (!w || (o == 0 && nx < WT)) continue;
+        const cuuint64_t c = o == 2 ? COUT : CIN;
+        const cuuint64_t dims[4] = {c, (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
+        const cuuint64_t strides[3] = {c * 2, (cuuint64_t)nx * c * 2, (cuuint64_t)nx * ny * c * 2};
+        const cuuint32_t box[4] = {(cuuint32_t)c, (cuuint32_t)w, 1, 1};
+        e = encode_bf16(&maps[o], 4, const_cast<void*>(o == 2 ? dy : x), dims, strides, box,
+                        c == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     }
     if (e == cudaSuccess) {
         k_conv3d_wgrad_tc<CIN, COUT><<<grid, WG_NTH, L::BYTES, st>>>(
-            xm, ym, use_tma, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy), static_cast<float*>(buf),
-            nx, ny, nz, err);
+            maps[0], maps[1], maps[2], static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy),
+            static_cast<float*>(buf), nx, ny, nz, err);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {

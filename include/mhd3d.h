@@ -320,10 +320,19 @@ int mhd3d_ensemble_set_stream(void* ens, void* stream);
  * the stream-ordered allocator (cudaMallocAsync on stream, freed after use)
  * and are added in a fixed order, so repeated calls give the same bits.  If
  * a bounded device-side wait gives up, dw and db receive NaN.
+ * mhd3d_conv3d_wgrad_ws: the same in the caller's workspace ws (device,
+ * 16-byte aligned, its contents are of no consequence; in use until the call's work
+ * has ended, so calls that may overlap take one each), of at most
+ * mhd3d_conv3d_wgrad_workspace(cin, cout) bytes for any grid on the current
+ * device; NULL for the allocator's.  That size is -1 for a pair (cin, cout)
+ * that is not supported.
  */
 int mhd3d_conv3d(int32_t cin, int32_t cout, const void* x, const void* w, const float* bias, const void* mask,
                  int32_t relu, void* y, float* yf, int32_t nx, int32_t ny, int32_t nz, int32_t* err, void* stream);
 int mhd3d_conv3d_wtranspose(int32_t cin, int32_t cout, const void* w, void* wt, void* stream);
+int64_t mhd3d_conv3d_wgrad_workspace(int32_t cin, int32_t cout);
+int mhd3d_conv3d_wgrad_ws(int32_t cin, int32_t cout, const void* x, const void* dy, float* dw, float* db, int32_t nx,
+                          int32_t ny, int32_t nz, void* ws, int64_t ws_bytes, void* stream);
 int mhd3d_conv3d_wgrad(int32_t cin, int32_t cout, const void* x, const void* dy, float* dw, float* db, int32_t nx,
                        int32_t ny, int32_t nz, void* stream);
 

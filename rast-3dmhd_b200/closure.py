@@ -10,7 +10,7 @@ stress tau_ij (6), heat flux q_i (3), EMF eps_i (3) -- divided by their scales.
 Every arithmetic step runs in the library (libmhd3d_gpu.so): coarsening and
 targets (mhd3d_coarsen), features, the tcgen05 convolutions and their input
 gradients (mhd3d_conv3d, mhd3d_conv3d_wtranspose), FP32 weight gradients
-(mhd3d_conv3d_wgrad), the loss and its gradient (mhd3d_closure_loss), Adam
+(mhd3d_conv3d_wgrad_ws), the loss and its gradient (mhd3d_closure_loss), Adam
 (mhd3d_adam), the closure tendencies (mhd3d_closure_tendency) and, for
 training on tendencies, their loss and adjoint (mhd3d_closure_tendency_loss,
 mhd3d_closure_tendency_adjoint).  torch provides device memory and streams.
@@ -69,6 +69,9 @@ class ClosureNet:
         self.in_scale = torch.ones(8, dtype=torch.float32, device="cuda")
         self.out_scale = torch.ones(12, dtype=torch.float32, device="cuda")
         self.err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        # partial sums of a weight gradient, of any layer and grid
+        self.ws = torch.empty(max(self.lib.mhd3d_conv3d_wgrad_workspace(ci, co) for ci, co, _ in LAYERS),
+                              dtype=torch.uint8, device="cuda")
 
     # -- passes ---------------------------------------------------------------
     def forward(self, feat, shape, stream):
@@ -95,8 +98,9 @@ class ClosureNet:
         nz, ny, nx = shape
         for li in range(len(LAYERS) - 1, -1, -1):
             cin, cout, _ = LAYERS[li]
-            _check(self.lib.mhd3d_conv3d_wgrad(cin, cout, _p(acts[li]), _p(dy), _p(self.dw[li]), _p(self.db[li]),
-                                               nx, ny, nz, C.c_void_p(stream)), "mhd3d_conv3d_wgrad")
+            _check(self.lib.mhd3d_conv3d_wgrad_ws(cin, cout, _p(acts[li]), _p(dy), _p(self.dw[li]), _p(self.db[li]),
+                                                  nx, ny, nz, _p(self.ws), self.ws.numel(), C.c_void_p(stream)),
+                   "mhd3d_conv3d_wgrad_ws")
             if li == 0:
                 break
             wt = torch.empty((cin, 27 * cout), dtype=torch.bfloat16, device="cuda")

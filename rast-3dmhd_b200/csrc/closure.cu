@@ -944,28 +944,34 @@ cudaError_t launch_conv_t(const void* x, const void* w, const float* bias, const
     return cudaGetLastError();
 }
 
-// the tensor-core weight gradient: one CTA per SM (a fixed grid of at most
-// the SM count over the segments), its partial rows in a stream-ordered
-// workspace, then the ordered reduction into dw, db
+// CTAs of the weight gradient: one per SM, at most one per segment
+int wgrad_grid(int ntile)
+{
+    int sms = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return ntile < sms ? ntile : sms;
+}
+
+// a partial row a CTA, and the error flag
+size_t wgrad_bytes(int cin, int cout, int grid)
+{
+    return (size_t)grid * ((size_t)cout * 27 * cin + cout) * sizeof(float) + 16;
+}
+
+// the tensor-core weight gradient: a fixed grid over the segments, its partial
+// rows in the workspace, then the ordered reduction into dw, db
 template <int CIN, int COUT>
-cudaError_t launch_wgrad_tc_t(const void* x, const void* dy, float* dw, float* db, int nx, int ny, int nz,
+cudaError_t launch_wgrad_tc_t(const void* x, const void* dy, float* dw, float* db, int nx, int ny, int nz, void* buf,
                               cudaStream_t st)
 {
     using L = WgLay<CIN, COUT>;
     static std::atomic<unsigned long long> attr{0};
-    cudaError_t ae = smem_attr_once(attr, reinterpret_cast<const void*>(k_conv3d_wgrad_tc<CIN, COUT>), L::BYTES);
-    if (ae != cudaSuccess) return ae;
-    int sms = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int ntile = ((nx + WT - 1) / WT) * ny * nz;
-    const int grid = ntile < sms ? ntile : sms;
-    const size_t stride = (size_t)COUT * 27 * CIN + COUT;
-    const size_t bytes = (size_t)grid * stride * sizeof(float) + 16;
-    void* buf = nullptr;
-    cudaError_t e = cudaMallocAsync(&buf, bytes, st);
+    cudaError_t e = smem_attr_once(attr, reinterpret_cast<const void*>(k_conv3d_wgrad_tc<CIN, COUT>), L::BYTES);
     if (e != cudaSuccess) return e;
-    int* err = reinterpret_cast<int*>(static_cast<char*>(buf) + (size_t)grid * stride * sizeof(float));
+    const int grid = wgrad_grid(((nx + WT - 1) / WT) * ny * nz);
+    const size_t stride = (size_t)COUT * 27 * CIN + COUT;
+    int* err = reinterpret_cast<int*>(static_cast<char*>(buf) + wgrad_bytes(CIN, COUT, grid) - 16);
     e = cudaMemsetAsync(err, 0, sizeof(int), st);
     // (channel, x, y, z) boxes: 64 voxels of x and dy, and of x what the row's last segment holds
     CUtensorMap maps[3];
@@ -992,8 +998,20 @@ cudaError_t launch_wgrad_tc_t(const void* x, const void* dy, float* dw, float* d
                                                                     dw, db, err);
         e = cudaGetLastError();
     }
-    const cudaError_t f = cudaFreeAsync(buf, st);
-    return e != cudaSuccess ? e : f;
+    return e;
+}
+
+cudaError_t launch_wgrad(int cin, int cout, const void* x, const void* dy, float* dw, float* db, int nx, int ny,
+                         int nz, void* buf, cudaStream_t st)
+{
+    if (cin == 16) return launch_wgrad_tc_t<16, 32>(x, dy, dw, db, nx, ny, nz, buf, st);
+    if (cout == 32) return launch_wgrad_tc_t<32, 32>(x, dy, dw, db, nx, ny, nz, buf, st);
+    return launch_wgrad_tc_t<32, 16>(x, dy, dw, db, nx, ny, nz, buf, st);
+}
+
+bool wgrad_shape(int cin, int cout)
+{
+    return (cin == 16 && cout == 32) || (cin == 32 && (cout == 32 || cout == 16));
 }
 
 }  // namespace clo
@@ -1021,18 +1039,36 @@ int mhd3d_conv3d(int32_t cin, int32_t cout, const void* x, const void* w, const 
     return e == cudaSuccess ? MHD3D_OK : MHD3D_ERR_CUDA;
 }
 
+int64_t mhd3d_conv3d_wgrad_workspace(int32_t cin, int32_t cout)
+{
+    return wgrad_shape(cin, cout) ? (int64_t)wgrad_bytes(cin, cout, wgrad_grid(INT32_MAX)) : -1;
+}
+
+// With no workspace given one is taken from the stream's allocator, whose
+// default pool returns its memory to the system at every synchronisation: the
+// first call after one then took 220 us of host time for a 24x16x8 layer, 15
+// with memory at hand.
+int mhd3d_conv3d_wgrad_ws(int32_t cin, int32_t cout, const void* x, const void* dy, float* dw, float* db, int32_t nx,
+                          int32_t ny, int32_t nz, void* ws, int64_t ws_bytes, void* stream)
+{
+    if (!x || !dy || !dw || nx <= 0 || ny <= 0 || nz <= 0) return MHD3D_ERR_ARG;
+    if (!aligned16(x) || !aligned16(dy) || !aligned16(ws) || !wgrad_shape(cin, cout)) return MHD3D_ERR_ARG;
+    const int grid = wgrad_grid(((nx + WT - 1) / WT) * ny * nz);
+    if (grid <= 0) return MHD3D_ERR_ARG;
+    const size_t bytes = wgrad_bytes(cin, cout, grid);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    void* own = nullptr;
+    if (ws && (ws_bytes < 0 || (size_t)ws_bytes < bytes)) return MHD3D_ERR_ARG;
+    if (!ws && cudaMallocAsync(&own, bytes, st) != cudaSuccess) return MHD3D_ERR_CUDA;
+    const cudaError_t e = launch_wgrad(cin, cout, x, dy, dw, db, nx, ny, nz, ws ? ws : own, st);
+    const cudaError_t f = own ? cudaFreeAsync(own, st) : cudaSuccess;
+    return e == cudaSuccess && f == cudaSuccess ? MHD3D_OK : MHD3D_ERR_CUDA;
+}
+
 int mhd3d_conv3d_wgrad(int32_t cin, int32_t cout, const void* x, const void* dy, float* dw, float* db, int32_t nx,
                        int32_t ny, int32_t nz, void* stream)
 {
-    if (!x || !dy || !dw || nx <= 0 || ny <= 0 || nz <= 0) return MHD3D_ERR_ARG;
-    if (!aligned16(x) || !aligned16(dy)) return MHD3D_ERR_ARG;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t e;
-    if (cin == 16 && cout == 32) e = launch_wgrad_tc_t<16, 32>(x, dy, dw, db, nx, ny, nz, st);
-    else if (cin == 32 && cout == 32) e = launch_wgrad_tc_t<32, 32>(x, dy, dw, db, nx, ny, nz, st);
-    else if (cin == 32 && cout == 16) e = launch_wgrad_tc_t<32, 16>(x, dy, dw, db, nx, ny, nz, st);
-    else return MHD3D_ERR_ARG;
-    return e == cudaSuccess ? MHD3D_OK : MHD3D_ERR_CUDA;
+    return mhd3d_conv3d_wgrad_ws(cin, cout, x, dy, dw, db, nx, ny, nz, nullptr, 0, stream);
 }
 
 int mhd3d_conv3d_wtranspose(int32_t cin, int32_t cout, const void* w, void* wt, void* stream)

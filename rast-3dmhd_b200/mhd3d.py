@@ -123,6 +123,9 @@ def gpu_lib() -> C.CDLL:
     lib.mhd3d_conv3d.argtypes = [i32, i32, vp, vp, vp, vp, i32, vp, vp, i32, i32, i32, vp, vp]
     lib.mhd3d_conv3d_wtranspose.argtypes = [i32, i32, vp, vp, vp]
     lib.mhd3d_conv3d_wgrad.argtypes = [i32, i32, vp, vp, vp, vp, i32, i32, i32, vp]
+    lib.mhd3d_conv3d_wgrad_ws.argtypes = [i32, i32, vp, vp, vp, vp, i32, i32, i32, vp, C.c_int64, vp]
+    lib.mhd3d_conv3d_wgrad_workspace.argtypes = [i32, i32]
+    lib.mhd3d_conv3d_wgrad_workspace.restype = C.c_int64
     lib.mhd3d_closure_set.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, C.c_float]
     lib.mhd3d_closure_status.argtypes = [vp, vp, vp, vp]
     lib.mhd3d_closure_set_bias.argtypes = [vp, vp]

@@ -12,7 +12,7 @@ reference checkout.
 
 The checkout's location comes from --src, else the environment variable
 MHD3D_REFERENCE_SRC, else the container's read-only mount.  With
---if-present a missing checkout is not an error (the GPU box has none).
+--if-present missing sources are not an error.
 """
 from __future__ import annotations
 
@@ -54,8 +54,8 @@ if __name__ == "__main__":
     ap.add_argument("--src", default=DEFAULT_SRC)
     ap.add_argument("--out", default=None)
     ap.add_argument("--if-present", action="store_true",
-                    help="exit quietly when the reference checkout is absent")
+                    help="exit quietly when the reference sources are absent")
     a = ap.parse_args()
-    if a.if_present and not os.path.isdir(a.src):
+    if a.if_present and not all(os.path.exists(os.path.join(a.src, f)) for f in ("3dmhdsub.f", "3dmhdparam.f")):
         sys.exit(0)
     print(build(a.src, a.out))

@@ -580,7 +580,7 @@ def run_closure(args, rank, world, local):
                            "fine_equivalent_note": "512^2*256 cells x (DT_coarse/DT_fine) per coarse step",
                            "parallelism": f"{world} independent replica(s), one per GPU, no collectives"},
                 "roofline": roof, "cpu_baseline": None,
-                "e2e": e2e, "gpu_launches": 12 * args.steps, "clocks": clk}
+                "e2e": e2e, "gpu_launches": 11 * args.steps, "clocks": clk}
         print(json.dumps(line), flush=True)
     sim.close()
     return 0
@@ -778,7 +778,7 @@ def main():
                            "parallelism": f"{world} independent replica(s), one per GPU, no collectives",
                            "last_dt": res["dt"], "nit": res["nit"]},
                 "roofline": roof, "cpu_baseline": cpu, "e2e": e2e,
-                "gpu_launches": 4 * args.steps, "clocks": clk}
+                "gpu_launches": 3 * args.steps, "clocks": clk}
     sim.close()
     # the metric's other half: the FP32+closure coarse run (default workload only)
     if not args.case and not args.grid and not args.no_closure:

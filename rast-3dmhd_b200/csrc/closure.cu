@@ -578,10 +578,11 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
 // apart (block j holds dx = 2-j; the leading offset of A is one voxel; blocks
 // beyond the third are unused lanes), the z taps the three planes of an input
 // row.  A row's last segment has boxes of its own width and only the K steps
-// that its voxels reach.  The loader warp runs up to WST segments ahead of the MMA thread.  The three accumulators (3*3*CIN columns)
-// stay in TMEM over all of a CTA's segments (a fixed set, in a fixed order);
-// each CTA writes its partial sums to a workspace row and a second kernel adds
-// the rows to dW in CTA order, so the result does not depend on timing.
+// that its voxels reach.  The loader warp runs up to WST segments ahead of
+// the MMA thread.  The three accumulators (3*3*CIN columns) stay in TMEM over
+// all of a CTA's segments (a fixed set, in a fixed order); each CTA writes
+// its partial sums to a workspace row and a second kernel adds the rows to dW
+// in CTA order, so the result does not depend on timing.
 //
 // Bound by L2 reads (42 KB a segment for 32 input channels) and the hand-offs
 // of three stages; 128x128x64, us: 16->32 117, 32->32 143, 32->16 129.  The

@@ -24,65 +24,40 @@
 namespace mhd3d {
 
 // per-column constants: HX*DXXDX, and HX*D2XXDX2 +- H2X*DXXDX**2, likewise y
-template <typename T>
 struct MarchCol {
-    T ax, xp, xm, ay, yp, ym;
+    double ax, xp, xm, ay, yp, ym;
 };
 
-template <typename T>
-__device__ __forceinline__ T mfma(T a, T b, T c);
-template <>
-__device__ __forceinline__ double mfma<double>(double a, double b, double c) { return fma(a, b, c); }
-template <>
-__device__ __forceinline__ float mfma<float>(float a, float b, float c) { return fmaf(a, b, c); }
-
-// a product that is rounded by itself (never part of an FMA)
-template <typename T>
-__device__ __forceinline__ T mmul(T a, T b);
-template <>
-__device__ __forceinline__ double mmul<double>(double a, double b) { return __dmul_rn(a, b); }
-template <>
-__device__ __forceinline__ float mmul<float>(float a, float b) { return __fmul_rn(a, b); }
-
-// T: arithmetic type; BG: fields are perturbations from per-plane backgrounds,
-// whose z differences join as constants of the plane; BWV, BS: row length and
-// field size of a plane slot in shared memory; PZ: a plane's constants.
-template <typename T, bool MAG, bool ROT, bool BG, int BWV, int BS, typename PZ>
+// BWV, BS: row length and field size of a plane slot in shared memory.
+template <bool MAG, bool ROT, int BWV, int BS>
 struct March {
-    // plane q-1: its cell, read again from its slot (b: without its background)
-    T ru, rv, rw, tt, ro, p, u, v, w;
-    T bx, by, bz;
+    // plane q-1: its cell, read again from its slot
+    double ru, rv, rw, tt, ro, p, u, v, w;
+    double bx, by, bz;
     // carried between arrivals for plane q-1
-    T ri;
-    T wx, wy, s;                                 // dw/dx, dw/dy, du/dx + dv/dy
-    T fu, fv, fw, fr, ft, heat, w1, w2, w3;      // what its right-hand side holds so far
-    T exz, eyz, wz, jx, jy;                      // du/dz + dw/dx, dv/dz + dw/dy, dw/dz, currents: without plane q
-    T dp;                                        // pressure less that of the plane above
+    double ri;
+    double wx, wy, s;                                 // dw/dx, dw/dy, du/dx + dv/dy
+    double fu, fv, fw, fr, ft, heat, w1, w2, w3;      // what its right-hand side holds so far
+    double exz, eyz, wz, jx, jy;                      // du/dz + dw/dx, dv/dz + dw/dy, dw/dz, currents: without plane q
+    double dp;                                        // pressure less that of the plane above
     // plane q
-    T nru, nrv, nrw, ntt, nro, nri, nu, nv, nw, np, nbx, nby, nbz;
-    T nwx, nwy, ns;
+    double nru, nrv, nrw, ntt, nro, nri, nu, nv, nw, np, nbx, nby, nbz;
+    double nwx, nwy, ns;
 
-    static __device__ __forceinline__ T ld(const T* __restrict__ raw, int f, int off) { return raw[f * BS + off]; }
-    // pressure, or its perturbation RHOb*T' + RO'*(Tb + T')
-    static __device__ __forceinline__ T pres(T ro_, T tt_, const PZ& z)
+    static __device__ __forceinline__ double ld(const double* __restrict__ raw, int f, int off)
     {
-        if constexpr (BG) return mfma<T>(ro_, z.ttb + tt_, z.rob * tt_);
-        else return mmul<T>(ro_, tt_);
+        return raw[f * BS + off];
     }
+    // the pressure, a product rounded by itself (never part of an FMA)
+    static __device__ __forceinline__ double pres(double ro_, double tt_) { return __dmul_rn(ro_, tt_); }
     // difference of two pressures of a plane
-    static __device__ __forceinline__ T dpres(T rop, T tp, T rom, T tm, const PZ& z)
+    static __device__ __forceinline__ double dpres(double rop, double tp, double rom, double tm)
     {
-        if constexpr (BG) return pres(rop, tp, z) - pres(rom, tm, z);
-        else return mfma<T>(rop, tp, -mmul<T>(rom, tm));
-    }
-    __device__ __forceinline__ T bfull(T b, T b0) const
-    {
-        if constexpr (BG) return b0 + b;
-        else return b;
+        return fma(rop, tp, -pres(rom, tm));
     }
 
     // the cell of plane q
-    __device__ __forceinline__ void cell(const T* __restrict__ raw, const T* __restrict__ rip, int o, const PZ& z)
+    __device__ __forceinline__ void cell(const double* __restrict__ raw, const double* __restrict__ rip, int o)
     {
         nru = ld(raw, F_RU, o);
         nrv = ld(raw, F_RV, o);
@@ -98,207 +73,189 @@ struct March {
         nu = nru * nri;
         nv = nrv * nri;
         nw = nrw * nri;
-        np = pres(nro, ntt, z);
+        np = pres(nro, ntt);
     }
 
-    __device__ __forceinline__ void arrive(const T* __restrict__ raw, const T* __restrict__ rip, int o,
-                                           const MarchCol<T>& c)
+    __device__ __forceinline__ void arrive(const double* __restrict__ raw, const double* __restrict__ rip, int o,
+                                           const MarchCol& c)
     {
-        const T rxp = rip[o + 1], rxm = rip[o - 1], ryp = rip[o + BWV], rym = rip[o - BWV];
-        nwx = mfma<T>(ld(raw, F_RW, o + 1), rxp, -ld(raw, F_RW, o - 1) * rxm) * c.ax;
-        nwy = mfma<T>(ld(raw, F_RW, o + BWV), ryp, -ld(raw, F_RW, o - BWV) * rym) * c.ay;
-        ns = mfma<T>(mfma<T>(ld(raw, F_RU, o + 1), rxp, -ld(raw, F_RU, o - 1) * rxm), c.ax,
-                     mfma<T>(ld(raw, F_RV, o + BWV), ryp, -ld(raw, F_RV, o - BWV) * rym) * c.ay);
+        const double rxp = rip[o + 1], rxm = rip[o - 1], ryp = rip[o + BWV], rym = rip[o - BWV];
+        nwx = fma(ld(raw, F_RW, o + 1), rxp, -ld(raw, F_RW, o - 1) * rxm) * c.ax;
+        nwy = fma(ld(raw, F_RW, o + BWV), ryp, -ld(raw, F_RW, o - BWV) * rym) * c.ay;
+        ns = fma(fma(ld(raw, F_RU, o + 1), rxp, -ld(raw, F_RU, o - 1) * rxm), c.ax,
+                     fma(ld(raw, F_RV, o + BWV), ryp, -ld(raw, F_RV, o - BWV) * rym) * c.ay);
     }
 
     // plane q-1's terms from plane q (z: the constants of plane q-1).  bot: it
     // is the bottom wall, whose d2BX/dz2, d2BY/dz2 are one-sided (l1, l2).
-    __device__ __forceinline__ void complete(const PZ& z, const MarchRun<T>& r, bool bot, T l1, T l2)
+    __device__ __forceinline__ void complete(const PlaneZ& z, const MarchRun& r, bool bot, double l1, double l2)
     {
-        const T du = nu - u, dv = nv - v, dw = nw - w, dt = ntt - tt;
-        fr = mfma<T>(rw - nrw, z.az, fr);
-        fu = mfma<T>(-nru * nw, z.az, fu);
-        fv = mfma<T>(-nrv * nw, z.az, fv);
-        fw = mfma<T>(mfma<T>(rw, w, -nrw * nw), z.az, fw);
-        fu = mfma<T>(z.ozp, du, mfma<T>(z.t13az, nwx, fu));
-        fv = mfma<T>(z.ozp, dv, mfma<T>(z.t13az, nwy, fv));
-        fw = mfma<T>(z.ozp, r.c43 * dw, mfma<T>(z.t13az, ns, fw));
-        if constexpr (BG) fw += mfma<T>(-(dp + (np - p)), z.az, mfma<T>(r.grav, ro, z.fw));
-        else fw = mfma<T>(r.grav, ro, mfma<T>(-(dp + mfma<T>(nro, ntt, -p)), z.az, fw));
-        exz = mfma<T>(du, z.az, exz);
-        eyz = mfma<T>(dv, z.az, eyz);
-        wz = mfma<T>(dw, z.az, wz);
-        ft = mfma<T>(dt, mfma<T>(ri * r.tmpc, z.kzp, -w * z.az), ft);
-        if constexpr (BG) ft = mfma<T>(-r.ocv * (z.ttb + tt), wz, ft);
-        else ft = mfma<T>(-r.ocv * tt, wz, ft);
-        heat = mfma<T>(r.tmpa, mfma<T>(exz, exz, mfma<T>(eyz, eyz, r.c43 * (wz * (wz - s)))), heat);
+        const double du = nu - u, dv = nv - v, dw = nw - w, dt = ntt - tt;
+        fr = fma(rw - nrw, z.az, fr);
+        fu = fma(-nru * nw, z.az, fu);
+        fv = fma(-nrv * nw, z.az, fv);
+        fw = fma(fma(rw, w, -nrw * nw), z.az, fw);
+        fu = fma(z.ozp, du, fma(z.t13az, nwx, fu));
+        fv = fma(z.ozp, dv, fma(z.t13az, nwy, fv));
+        fw = fma(z.ozp, r.c43 * dw, fma(z.t13az, ns, fw));
+        fw = fma(r.grav, ro, fma(-(dp + fma(nro, ntt, -p)), z.az, fw));
+        exz = fma(du, z.az, exz);
+        eyz = fma(dv, z.az, eyz);
+        wz = fma(dw, z.az, wz);
+        ft = fma(dt, fma(ri * r.tmpc, z.kzp, -w * z.az), ft);
+        ft = fma(-r.ocv * tt, wz, ft);
+        heat = fma(r.tmpa, fma(exz, exz, fma(eyz, eyz, r.c43 * (wz * (wz - s)))), heat);
         if (MAG) {
-            const T dbx = nbx - bx, dby = nby - by, dbz = nbz - bz;
-            const T fbx = bfull(bx, bgx(z)), fby = bfull(by, bgy(z)), fbz = bfull(bz, bgz(z));
-            jy = mfma<T>(dbx, z.az, jy);
-            jx = mfma<T>(dby, z.az, jx);
+            const double dbx = nbx - bx, dby = nby - by, dbz = nbz - bz;
+            jy = fma(dbx, z.az, jy);
+            jx = fma(dby, z.az, jx);
             w1 += bot ? l1 : z.mzp * dbx;
             w2 += bot ? l2 : z.mzp * dby;
-            w1 = mfma<T>(fbz, exz, mfma<T>(-fbx, wz, mfma<T>(-w, jy, w1)));
-            w2 = mfma<T>(fbz, eyz, mfma<T>(-fby, wz, mfma<T>(-w, jx, w2)));
-            w3 = mfma<T>(dbz, mfma<T>(-w, z.az, z.mzp), w3);
-            const T oy = r.obeta * jy, ox = r.obeta * jx;
-            fu = mfma<T>(fbz, oy, fu);
-            fv = mfma<T>(fbz, ox, fv);
-            fw -= mfma<T>(fbx, oy, fby * ox);
-            heat = mfma<T>(r.tmpm, mfma<T>(jx, jx, jy * jy), heat);
+            w1 = fma(bz, exz, fma(-bx, wz, fma(-w, jy, w1)));
+            w2 = fma(bz, eyz, fma(-by, wz, fma(-w, jx, w2)));
+            w3 = fma(dbz, fma(-w, z.az, z.mzp), w3);
+            const double oy = r.obeta * jy, ox = r.obeta * jx;
+            fu = fma(bz, oy, fu);
+            fv = fma(bz, ox, fv);
+            fw -= fma(bx, oy, by * ox);
+            heat = fma(r.tmpm, fma(jx, jx, jy * jy), heat);
         }
-        ft = mfma<T>(ri, heat, ft);
+        ft = fma(ri, heat, ft);
     }
-
-    static __device__ __forceinline__ T bgx(const PZ& z) { if constexpr (BG) return z.bx; else return T(0); }
-    static __device__ __forceinline__ T bgy(const PZ& z) { if constexpr (BG) return z.by; else return T(0); }
-    static __device__ __forceinline__ T bgz(const PZ& z) { if constexpr (BG) return z.bz; else return T(0); }
 
     // plane q's x, y terms and its terms from plane q-1 (z: the constants of
     // plane q).  top: it is the top wall, as in complete().
-    __device__ __forceinline__ void begin(const T* __restrict__ raw, const T* __restrict__ rip, int o, const PZ& z,
-                                          const T* __restrict__ rawk, const PZ& zk,
-                                          const MarchCol<T>& c, const MarchRun<T>& r, bool top, T rwt, T wt, T l1, T l2)
+    __device__ __forceinline__ void begin(const double* __restrict__ raw, const double* __restrict__ rip, int o,
+                                          const PlaneZ& z, const double* __restrict__ rawk, const MarchCol& c,
+                                          const MarchRun& r, bool top, double rwt, double wt, double l1, double l2)
     {
-        cell(raw, rip, o, z);
-        recall(rawk, o, zk);
+        cell(raw, rip, o);
+        recall(rawk, o);
         if (top) {   // one-sided dRW/dz, dw/dz
             rw = rwt;
             w = wt;
         }
-        const T du = nu - u, dv = nv - v, dw = nw - w, dt = ntt - tt;
-        T gu, gv, gw, gr, gt, gh;
+        const double du = nu - u, dv = nv - v, dw = nw - w, dt = ntt - tt;
+        double gu, gv, gw, gr, gt, gh;
         // terms from the plane above, and dw/dz, strain and current sums that start with it
         gr = (rw - nrw) * z.az;
-        gu = mfma<T>(ru * w, z.az, mfma<T>(z.ozm, du, -z.t13az * wx));
-        gv = mfma<T>(rv * w, z.az, mfma<T>(z.ozm, dv, -z.t13az * wy));
+        gu = fma(ru * w, z.az, fma(z.ozm, du, -z.t13az * wx));
+        gv = fma(rv * w, z.az, fma(z.ozm, dv, -z.t13az * wy));
         dp = np - p;
-        gw = mfma<T>(mfma<T>(rw, w, -nrw * nw), z.az, mfma<T>(z.ozm, r.c43 * dw, -z.t13az * s));
-        const T q = nri * r.tmpc;
-        gt = dt * mfma<T>(q, z.kzm, -nw * z.az);
-        exz = mfma<T>(du, z.az, nwx);
-        eyz = mfma<T>(dv, z.az, nwy);
+        gw = fma(fma(rw, w, -nrw * nw), z.az, fma(z.ozm, r.c43 * dw, -z.t13az * s));
+        const double q = nri * r.tmpc;
+        gt = dt * fma(q, z.kzm, -nw * z.az);
+        exz = fma(du, z.az, nwx);
+        eyz = fma(dv, z.az, nwy);
         wz = dw * z.az;
-        T tf = ntt;   // full temperature
-        if constexpr (BG) {
-            gt = mfma<T>(q, z.kbg, mfma<T>(-nw, z.tzaz, gt));
-            tf += z.ttb;
-        }
-        gt = mfma<T>(-r.ocv * tf, ns, gt);
+        gt = fma(-r.ocv * ntt, ns, gt);
         if (ROT) {
-            gu = mfma<T>(r.omz, nrv, gu);
-            gv = mfma<T>(r.omx, nrw, mfma<T>(-r.omz, nru, gv));
-            gw = mfma<T>(-r.omx, nrv, gw);
+            gu = fma(r.omz, nrv, gu);
+            gv = fma(r.omx, nrw, fma(-r.omz, nru, gv));
+            gw = fma(-r.omx, nrv, gw);
         }
-        T lt;   // x, y part of the Laplacian of T
-        T vx, ux;
+        double lt;   // x, y part of the Laplacian of T
+        double vx, ux;
         {   // x
-            const T rxp = rip[o + 1], rxm = rip[o - 1];
-            const T rup = ld(raw, F_RU, o + 1), rum = ld(raw, F_RU, o - 1);
-            const T rvp = ld(raw, F_RV, o + 1), rvm = ld(raw, F_RV, o - 1);
-            const T rwp = ld(raw, F_RW, o + 1), rwm = ld(raw, F_RW, o - 1);
-            const T tp = ld(raw, F_TT, o + 1), tm = ld(raw, F_TT, o - 1);
-            const T dpx = dpres(ld(raw, F_RO, o + 1), tp, ld(raw, F_RO, o - 1), tm, z);
-            const T vp = rvp * rxp, vm = rvm * rxm, uxp = rup * rxp, uxm = rum * rxm, wxp = rwp * rxp, wxm = rwm * rxm;
-            gr = mfma<T>(-(rup - rum), c.ax, gr);
-            gu = mfma<T>(-mfma<T>(rup, uxp, mfma<T>(-rum, uxm, dpx)), c.ax, gu);
-            gv = mfma<T>(-mfma<T>(rvp, uxp, -rvm * uxm), c.ax, gv);
-            gw = mfma<T>(-mfma<T>(rwp, uxp, -rwm * uxm), c.ax, gw);
-            gu = mfma<T>(r.ore43, mfma<T>(uxp - nu, c.xp, (nu - uxm) * c.xm), gu);
-            gv = mfma<T>(r.ore, mfma<T>(vp - nv, c.xp, (nv - vm) * c.xm), gv);
-            gw = mfma<T>(r.ore, mfma<T>(wxp - nw, c.xp, (nw - wxm) * c.xm), gw);
-            gt = mfma<T>(-nu, (tp - tm) * c.ax, gt);
-            lt = mfma<T>(tp - ntt, c.xp, (ntt - tm) * c.xm);
+            const double rxp = rip[o + 1], rxm = rip[o - 1];
+            const double rup = ld(raw, F_RU, o + 1), rum = ld(raw, F_RU, o - 1);
+            const double rvp = ld(raw, F_RV, o + 1), rvm = ld(raw, F_RV, o - 1);
+            const double rwp = ld(raw, F_RW, o + 1), rwm = ld(raw, F_RW, o - 1);
+            const double tp = ld(raw, F_TT, o + 1), tm = ld(raw, F_TT, o - 1);
+            const double dpx = dpres(ld(raw, F_RO, o + 1), tp, ld(raw, F_RO, o - 1), tm);
+            const double vp = rvp * rxp, vm = rvm * rxm, uxp = rup * rxp, uxm = rum * rxm;
+            const double wxp = rwp * rxp, wxm = rwm * rxm;
+            gr = fma(-(rup - rum), c.ax, gr);
+            gu = fma(-fma(rup, uxp, fma(-rum, uxm, dpx)), c.ax, gu);
+            gv = fma(-fma(rvp, uxp, -rvm * uxm), c.ax, gv);
+            gw = fma(-fma(rwp, uxp, -rwm * uxm), c.ax, gw);
+            gu = fma(r.ore43, fma(uxp - nu, c.xp, (nu - uxm) * c.xm), gu);
+            gv = fma(r.ore, fma(vp - nv, c.xp, (nv - vm) * c.xm), gv);
+            gw = fma(r.ore, fma(wxp - nw, c.xp, (nw - wxm) * c.xm), gw);
+            gt = fma(-nu, (tp - tm) * c.ax, gt);
+            lt = fma(tp - ntt, c.xp, (ntt - tm) * c.xm);
             ux = (uxp - uxm) * c.ax;
             vx = (vp - vm) * c.ax;
         }
-        T uy, vy;
+        double uy, vy;
         {   // y
-            const T ryp = rip[o + BWV], rym = rip[o - BWV];
-            const T rup = ld(raw, F_RU, o + BWV), rum = ld(raw, F_RU, o - BWV);
-            const T rvp = ld(raw, F_RV, o + BWV), rvm = ld(raw, F_RV, o - BWV);
-            const T rwp = ld(raw, F_RW, o + BWV), rwm = ld(raw, F_RW, o - BWV);
-            const T tp = ld(raw, F_TT, o + BWV), tm = ld(raw, F_TT, o - BWV);
-            const T dpy = dpres(ld(raw, F_RO, o + BWV), tp, ld(raw, F_RO, o - BWV), tm, z);
-            const T up = rup * ryp, um = rum * rym, vyp = rvp * ryp, vym = rvm * rym, wyp = rwp * ryp, wym = rwm * rym;
-            gr = mfma<T>(-(rvp - rvm), c.ay, gr);
-            gu = mfma<T>(-mfma<T>(rup, vyp, -rum * vym), c.ay, gu);
-            gv = mfma<T>(-mfma<T>(rvp, vyp, mfma<T>(-rvm, vym, dpy)), c.ay, gv);
-            gw = mfma<T>(-mfma<T>(rwp, vyp, -rwm * vym), c.ay, gw);
-            gu = mfma<T>(r.ore, mfma<T>(up - nu, c.yp, (nu - um) * c.ym), gu);
-            gv = mfma<T>(r.ore43, mfma<T>(vyp - nv, c.yp, (nv - vym) * c.ym), gv);
-            gw = mfma<T>(r.ore, mfma<T>(wyp - nw, c.yp, (nw - wym) * c.ym), gw);
-            gt = mfma<T>(-nv, (tp - tm) * c.ay, gt);
-            lt += mfma<T>(tp - ntt, c.yp, (ntt - tm) * c.ym);
+            const double ryp = rip[o + BWV], rym = rip[o - BWV];
+            const double rup = ld(raw, F_RU, o + BWV), rum = ld(raw, F_RU, o - BWV);
+            const double rvp = ld(raw, F_RV, o + BWV), rvm = ld(raw, F_RV, o - BWV);
+            const double rwp = ld(raw, F_RW, o + BWV), rwm = ld(raw, F_RW, o - BWV);
+            const double tp = ld(raw, F_TT, o + BWV), tm = ld(raw, F_TT, o - BWV);
+            const double dpy = dpres(ld(raw, F_RO, o + BWV), tp, ld(raw, F_RO, o - BWV), tm);
+            const double up = rup * ryp, um = rum * rym, vyp = rvp * ryp, vym = rvm * rym;
+            const double wyp = rwp * ryp, wym = rwm * rym;
+            gr = fma(-(rvp - rvm), c.ay, gr);
+            gu = fma(-fma(rup, vyp, -rum * vym), c.ay, gu);
+            gv = fma(-fma(rvp, vyp, fma(-rvm, vym, dpy)), c.ay, gv);
+            gw = fma(-fma(rwp, vyp, -rwm * vym), c.ay, gw);
+            gu = fma(r.ore, fma(up - nu, c.yp, (nu - um) * c.ym), gu);
+            gv = fma(r.ore43, fma(vyp - nv, c.yp, (nv - vym) * c.ym), gv);
+            gw = fma(r.ore, fma(wyp - nw, c.yp, (nw - wym) * c.ym), gw);
+            gt = fma(-nv, (tp - tm) * c.ay, gt);
+            lt += fma(tp - ntt, c.yp, (ntt - tm) * c.ym);
             uy = (up - um) * c.ay;
             vy = (vyp - vym) * c.ay;
         }
-        gt = mfma<T>(q * z.rka, lt, gt);
+        gt = fma(q * z.rka, lt, gt);
         {   // corners: d2v/dxdy, d2u/dxdy
-            const T rpp = rip[o + BWV + 1], rmp = rip[o + BWV - 1], rpm = rip[o - BWV + 1], rmm = rip[o - BWV - 1];
-            const T sxy = r.t13 * (c.ax * c.ay);
-            const T vv = mfma<T>(ld(raw, F_RV, o + BWV + 1), rpp, -ld(raw, F_RV, o + BWV - 1) * rmp)
-                       - mfma<T>(ld(raw, F_RV, o - BWV + 1), rpm, -ld(raw, F_RV, o - BWV - 1) * rmm);
-            const T uu = mfma<T>(ld(raw, F_RU, o + BWV + 1), rpp, -ld(raw, F_RU, o + BWV - 1) * rmp)
-                       - mfma<T>(ld(raw, F_RU, o - BWV + 1), rpm, -ld(raw, F_RU, o - BWV - 1) * rmm);
-            gu = mfma<T>(sxy, vv, gu);
-            gv = mfma<T>(sxy, uu, gv);
+            const double rpp = rip[o + BWV + 1], rmp = rip[o + BWV - 1], rpm = rip[o - BWV + 1], rmm = rip[o - BWV - 1];
+            const double sxy = r.t13 * (c.ax * c.ay);
+            const double vv = fma(ld(raw, F_RV, o + BWV + 1), rpp, -ld(raw, F_RV, o + BWV - 1) * rmp)
+                       - fma(ld(raw, F_RV, o - BWV + 1), rpm, -ld(raw, F_RV, o - BWV - 1) * rmm);
+            const double uu = fma(ld(raw, F_RU, o + BWV + 1), rpp, -ld(raw, F_RU, o + BWV - 1) * rmp)
+                       - fma(ld(raw, F_RU, o - BWV + 1), rpm, -ld(raw, F_RU, o - BWV - 1) * rmm);
+            gu = fma(sxy, vv, gu);
+            gv = fma(sxy, uu, gv);
         }
         {
-            const T e = uy + vx;
-            gh = r.tmpa * mfma<T>(e, e, r.c43 * mfma<T>(ns, ns, T(-3) * ux * vy));
+            const double e = uy + vx;
+            gh = r.tmpa * fma(e, e, r.c43 * fma(ns, ns, -3.0 * ux * vy));
         }
         if (MAG) {
-            const T fbx = bfull(nbx, bgx(z)), fby = bfull(nby, bgy(z)), fbz = bfull(nbz, bgz(z));
-            const T dbx = nbx - bx, dby = nby - by, dbz = nbz - bz;
-            T g1 = top ? l1 : z.mzm * dbx, g2 = top ? l2 : z.mzm * dby, g3 = dbz * mfma<T>(-nw, z.az, z.mzm);
-            T cy = dbx * z.az, cx = dby * z.az;   // currents without d/dx BZ, d/dy BZ
-            if constexpr (BG) {
-                g1 += z.ml1;
-                g2 += z.ml2;
-                g3 += mfma<T>(-nw, z.bzz, z.ml3);
-                cy += z.bxz;
-                cx += z.byz;
-            }
-            T lx, jz;
+            const double dbx = nbx - bx, dby = nby - by, dbz = nbz - bz;
+            double g1 = top ? l1 : z.mzm * dbx, g2 = top ? l2 : z.mzm * dby, g3 = dbz * fma(-nw, z.az, z.mzm);
+            double cy = dbx * z.az, cx = dby * z.az;   // currents without d/dx BZ, d/dy BZ
+            double lx, jz;
             {   // x
-                const T b1p = ld(raw, F_BX, o + 1), b1m = ld(raw, F_BX, o - 1);
-                const T b2p = ld(raw, F_BY, o + 1), b2m = ld(raw, F_BY, o - 1);
-                const T b3p = ld(raw, F_BZ, o + 1), b3m = ld(raw, F_BZ, o - 1);
-                const T d2 = (b2p - b2m) * c.ax, d3 = (b3p - b3m) * c.ax;
-                lx = mfma<T>(b1p - nbx, c.xp, (nbx - b1m) * c.xm);
-                g1 = mfma<T>(r.orm, lx, mfma<T>(-nu, (b1p - b1m) * c.ax, g1));
-                lx = mfma<T>(b2p - nby, c.xp, (nby - b2m) * c.xm);
-                g2 = mfma<T>(r.orm, lx, mfma<T>(-nu, d2, g2));
-                lx = mfma<T>(b3p - nbz, c.xp, (nbz - b3m) * c.xm);
-                g3 = mfma<T>(r.orm, lx, mfma<T>(-nu, d3, g3));
-                g1 = mfma<T>(-nw, d3, g1);
+                const double b1p = ld(raw, F_BX, o + 1), b1m = ld(raw, F_BX, o - 1);
+                const double b2p = ld(raw, F_BY, o + 1), b2m = ld(raw, F_BY, o - 1);
+                const double b3p = ld(raw, F_BZ, o + 1), b3m = ld(raw, F_BZ, o - 1);
+                const double d2 = (b2p - b2m) * c.ax, d3 = (b3p - b3m) * c.ax;
+                lx = fma(b1p - nbx, c.xp, (nbx - b1m) * c.xm);
+                g1 = fma(r.orm, lx, fma(-nu, (b1p - b1m) * c.ax, g1));
+                lx = fma(b2p - nby, c.xp, (nby - b2m) * c.xm);
+                g2 = fma(r.orm, lx, fma(-nu, d2, g2));
+                lx = fma(b3p - nbz, c.xp, (nbz - b3m) * c.xm);
+                g3 = fma(r.orm, lx, fma(-nu, d3, g3));
+                g1 = fma(-nw, d3, g1);
                 cy -= d3;
                 jz = -d2;
             }
             {   // y
-                const T b1p = ld(raw, F_BX, o + BWV), b1m = ld(raw, F_BX, o - BWV);
-                const T b2p = ld(raw, F_BY, o + BWV), b2m = ld(raw, F_BY, o - BWV);
-                const T b3p = ld(raw, F_BZ, o + BWV), b3m = ld(raw, F_BZ, o - BWV);
-                const T d1 = (b1p - b1m) * c.ay, d3 = (b3p - b3m) * c.ay;
-                lx = mfma<T>(b1p - nbx, c.yp, (nbx - b1m) * c.ym);
-                g1 = mfma<T>(r.orm, lx, mfma<T>(-nv, d1, g1));
-                lx = mfma<T>(b2p - nby, c.yp, (nby - b2m) * c.ym);
-                g2 = mfma<T>(r.orm, lx, mfma<T>(-nv, (b2p - b2m) * c.ay, g2));
-                lx = mfma<T>(b3p - nbz, c.yp, (nbz - b3m) * c.ym);
-                g3 = mfma<T>(r.orm, lx, mfma<T>(-nv, d3, g3));
-                g2 = mfma<T>(-nw, d3, g2);
+                const double b1p = ld(raw, F_BX, o + BWV), b1m = ld(raw, F_BX, o - BWV);
+                const double b2p = ld(raw, F_BY, o + BWV), b2m = ld(raw, F_BY, o - BWV);
+                const double b3p = ld(raw, F_BZ, o + BWV), b3m = ld(raw, F_BZ, o - BWV);
+                const double d1 = (b1p - b1m) * c.ay, d3 = (b3p - b3m) * c.ay;
+                lx = fma(b1p - nbx, c.yp, (nbx - b1m) * c.ym);
+                g1 = fma(r.orm, lx, fma(-nv, d1, g1));
+                lx = fma(b2p - nby, c.yp, (nby - b2m) * c.ym);
+                g2 = fma(r.orm, lx, fma(-nv, (b2p - b2m) * c.ay, g2));
+                lx = fma(b3p - nbz, c.yp, (nbz - b3m) * c.ym);
+                g3 = fma(r.orm, lx, fma(-nv, d3, g3));
+                g2 = fma(-nw, d3, g2);
                 cx -= d3;
                 jz += d1;
             }
-            g1 = mfma<T>(fby, uy, mfma<T>(-fbx, vy, mfma<T>(-fbz, nwx, g1)));
-            g2 = mfma<T>(fbx, vx, mfma<T>(-fby, ux, mfma<T>(-fbz, nwy, g2)));
-            g3 = mfma<T>(fbx, nwx, mfma<T>(fby, nwy, mfma<T>(-fbz, ns, g3)));
-            const T oz = r.obeta * jz;
-            gu = mfma<T>(fby, oz, gu);
-            gv = mfma<T>(-fbx, oz, gv);
-            gh = mfma<T>(r.tmpm * jz, jz, gh);
+            g1 = fma(nby, uy, fma(-nbx, vy, fma(-nbz, nwx, g1)));
+            g2 = fma(nbx, vx, fma(-nby, ux, fma(-nbz, nwy, g2)));
+            g3 = fma(nbx, nwx, fma(nby, nwy, fma(-nbz, ns, g3)));
+            const double oz = r.obeta * jz;
+            gu = fma(nby, oz, gu);
+            gv = fma(-nbx, oz, gv);
+            gh = fma(r.tmpm * jz, jz, gh);
             w1 = g1;
             w2 = g2;
             w3 = g3;
@@ -316,15 +273,16 @@ struct March {
     // one-sided d2B/dz2 on a wall (3dmhdsub.f:1510-1513 and the like) without the
     // part the march adds for the neighbour inside: b0 the wall, b1..b3 the
     // planes inside it, sg +1 on the top wall, -1 on the bottom wall
-    static __device__ __forceinline__ T wall_d2(const PZ& z, T sg, T b0, T b1, T b2, T b3)
+    static __device__ __forceinline__ double wall_d2(const PlaneZ& z, double sg, double b0, double b1, double b2,
+                                                     double b3)
     {
-        const T B = sg * (T(0.5) * (z.mzp + z.mzm)), C = T(0.5) * (z.mzp - z.mzm);
-        const T d1 = b1 - b0, d2 = b2 - b1, d3 = b3 - b2;
-        return mfma<T>(T(2) * d1 - d2, B, (T(3) * (d2 - d1) - d3) * C);
+        const double B = sg * (0.5 * (z.mzp + z.mzm)), C = 0.5 * (z.mzp - z.mzm);
+        const double d1 = b1 - b0, d2 = b2 - b1, d3 = b3 - b2;
+        return fma(2.0 * d1 - d2, B, (3.0 * (d2 - d1) - d3) * C);
     }
 
-    // the cell of plane q-1, from its slot (z: its constants)
-    __device__ __forceinline__ void recall(const T* __restrict__ raw, int o, const PZ& z)
+    // the cell of plane q-1, from its slot
+    __device__ __forceinline__ void recall(const double* __restrict__ raw, int o)
     {
         ru = ld(raw, F_RU, o);
         rv = ld(raw, F_RV, o);
@@ -339,11 +297,11 @@ struct March {
         u = ru * ri;
         v = rv * ri;
         w = rw * ri;
-        p = pres(ro, tt, z);
+        p = pres(ro, tt);
     }
 
     // plane q becomes the carried plane (rq: its 1/RO)
-    __device__ __forceinline__ void shift(T rq)
+    __device__ __forceinline__ void shift(double rq)
     {
         ri = rq;
         wx = nwx;

@@ -60,7 +60,7 @@ struct Handle {
     float* bg32 = nullptr;        // 2 x NZ: RHOb, Tb (FP32)
     PlaneBg* pb = nullptr;        // per interior plane
     PlaneZ* pz = nullptr;         // per U plane (FP64)
-    MarchRun<double> run{};
+    MarchRun run{};
     std::vector<double> faz_h, fbz_h, fcz_h;   // host copies of the z stencil factors
     std::vector<double> rka_h, dka_h, ddz_h;   // and of RKAPA, DKAPA, DDZ
     ColC* cxy = nullptr;                       // FP32 column constants: NX in x, then NY in y
@@ -1346,7 +1346,7 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
         f.obeta = (float)p->obeta; f.tmpm = (float)s.tmp_m; f.ogamma = (float)(1.0 / p->gamma);
         f.gamma = (float)p->gamma; f.cw3 = (float)s.cw3;
     }
-    h->run = MarchRun<double>{p->grav, p->ore, p->c43, p->ore * p->c43, s.tmp_13, s.tmp_a, s.tmp_cond, p->ocv,
+    h->run = MarchRun{p->grav, p->ore, p->c43, p->ore * p->c43, s.tmp_13, s.tmp_a, s.tmp_cond, p->ocv,
                               p->omx, p->omz, p->orm, p->obeta, s.tmp_m};
     if (!h->f32) {
         std::vector<PlaneZ> pz(NZ);

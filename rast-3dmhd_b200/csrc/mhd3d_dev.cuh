@@ -117,9 +117,8 @@ struct alignas(16) PlaneZ {
 };
 
 // run constants of the march (MarchRun in its order)
-template <typename T>
 struct MarchRun {
-    T grav, ore, c43, ore43, t13, tmpa, tmpc, ocv, omx, omz, orm, obeta, tmpm;
+    double grav, ore, c43, ore43, t13, tmpa, tmpc, ocv, omx, omz, orm, obeta, tmpm;
 };
 
 struct StageArgs {
@@ -135,7 +134,7 @@ struct StageArgs {
     Metrics m;
     Scalars s;
     const PlaneZ* pz;       // per U plane (FMA build)
-    MarchRun<double> run;
+    MarchRun run;
     size_t uf, uz;          // U: doubles per field, per plane
     size_t zf, zz;          // Z: doubles per field, per plane
     int upitch, zpitch;

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
 {
     using L = Lay<MAG, STAGE>;
     constexpr int NR = L::NR;
-    using Mc = March<double, MAG, ROT, false, BW, BSLOT, PlaneZ>;
+    using Mc = March<MAG, ROT, BW, BSLOT>;
     constexpr int NF = L::NF;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // 128-byte aligned base, formed by pointer arithmetic on the shared array
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     const Control* ctl = a.ctl;
     const Scalars& s = a.s;
     const Metrics& m = a.m;
-    const MarchRun<double>& run = a.run;
+    const MarchRun& run = a.run;
     const int npx = s.npx, npy = s.npy, npz = s.npz;
     const int tid = threadIdx.x;
     const int tx = tid % TX, ty = tid / TX;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     const double cu = STAGE == 1 ? s.gam1 * DT : STAGE == 2 ? s.gam2 * DT : s.gam3 * DT;
     const double cz = s.zeta2 * DT;
     const double C13 = s.c13, C23 = s.c23, C43 = s.c43;
-    MarchCol<double> col;
+    MarchCol col;
     {
         const int i = active ? gi + 1 : 1, j = active ? gj + 1 : 1;
         col.ax = m.fax[i];
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                 const PlaneZ& zk = *reinterpret_cast<const PlaneZ*>(rawk + L::REC);
                 c.arrive(raw, rip, o, col);
                 if (q > k0) {
-                    c.cell(raw, rip, o, zq);
-                    c.recall(rawk, o, zk);
+                    c.cell(raw, rip, o);
+                    c.recall(rawk, o);
                     const bool top = (k == 0), bot = (k == npz - 1), wall = top || bot;
                     const double ghost = c.nri;
                     double l1 = 0.0, l2 = 0.0;
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                             l2 = Mc::wall_d2(zq, 1.0, raw[F_BY * BSLOT + o], u[F_BY * a.uf], u2[F_BY * a.uf], u3[F_BY * a.uf]);
                         }
                     }
-                    c.begin(raw, rip, o, zq, rawk, zk, col, run, top, rwt, wt, l1, l2);
+                    c.begin(raw, rip, o, zq, rawk, col, run, top, rwt, wt, l1, l2);
                 }
                 c.shift(rip[o]);
             } else if (STAGE >= 2 && q > k0) {

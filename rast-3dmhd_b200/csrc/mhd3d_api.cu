@@ -260,30 +260,24 @@ __global__ void k_pack_interior32(const float* __restrict__ f, double* __restric
 }
 
 // ---- horizontally averaged profiles (HORIZONTAL_MEAN, 3dmhdsub.f:3143-3223) ----
-// One block per interior plane; per-thread partial sums in a fixed order, then a
-// fixed tree, so the result is deterministic.  Per-cell formulas follow the
-// reference's flux diagnostics (1651-1661).
-constexpr int PROF_THREADS = 256;
+// Per-cell formulas follow the reference's flux diagnostics (1651-1661); sums
+// are FP64, in a fixed order.  Bound by the read of the state: a plane's rows
+// are shared by enough CTAs to fill the device, and every field is read once.
+// FCONV needs the deviations from the plane's mean temperature, known only at
+// the end: the sums take them from the plane's first cell (as small), and
+// the mean of RW corrects for the difference.
+// A call on 256x256x128, host and copy included: FP64 143 us, FP32 130; one
+// CTA a plane with a second pass for FCONV took 585 and 744.  3 CTAs an SM
+// (no spills) 177 and 152.
+constexpr int PROF_WARPS = 8, PROF_SUMS = 7, PROF_CTAS = 4;
 
-__device__ __forceinline__ double block_sum(double v, double* red)
+template <bool F32, bool MAG>
+__global__ void __launch_bounds__(32 * PROF_WARPS, PROF_CTAS)
+k_profiles(const void* __restrict__ ubuf, const double* __restrict__ bgd, double* __restrict__ part, int npx, int npy,
+           int npz, int upitch, size_t uz, size_t uf)
 {
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int w = PROF_THREADS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    const double r = red[0];
-    __syncthreads();
-    return r;
-}
-
-template <bool F32>
-__global__ void __launch_bounds__(PROF_THREADS) k_profiles(const void* __restrict__ ubuf, const double* __restrict__ bgd,
-                                                           double* __restrict__ out, int npx, int npy, int npz,
-                                                           int upitch, size_t uz, size_t uf, int lmag)
-{
-    __shared__ double red[PROF_THREADS];
+    __shared__ double red[PROF_WARPS][PROF_SUMS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x;   // interior plane, Fortran K = k+2
     const int K0 = k + 1;       // U plane index
     const size_t NZ = (size_t)npz + 2;
@@ -295,53 +289,67 @@ __global__ void __launch_bounds__(PROF_THREADS) k_profiles(const void* __restric
         }
         return reinterpret_cast<const double*>(ubuf)[(size_t)f * uf + off];
     };
-    const int n = npx * npy;
-    double sro = 0.0, stt = 0.0, ske = 0.0, sen = 0.0, sme = 0.0;
-    for (int q = threadIdx.x; q < n; q += PROF_THREADS) {
-        const int i = q % npx, j = q / npx;
-        const size_t off = (size_t)K0 * uz + (size_t)(j + 1) * upitch + (i + 1);
-        const double ro = val(F_RO, off), tt = val(F_TT, off);
-        const double ri = 1.0 / ro;
-        const double u = val(F_RU, off) * ri, v = val(F_RV, off) * ri, w = val(F_RW, off) * ri;
-        sro += ro;
-        stt += tt;
-        ske += 0.5 * ro * (u * u + v * v + w * w);
-        sen += 2.5 * ro * tt;
-        if (lmag) {
-            const double bx = val(F_BX, off), by = val(F_BY, off), bz = val(F_BZ, off);
-            sme += 0.5 * (bx * bx + by * by + bz * bz);
+    const size_t plane = (size_t)K0 * uz + upitch + 1;
+    const double t0 = val(F_TT, plane);
+    double a[PROF_SUMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // RO, TT, KE, enthalpy, FCONV, ME, RW
+    for (int j = blockIdx.y * PROF_WARPS + warp; j < npy; j += gridDim.y * PROF_WARPS)
+        for (int i = lane; i < npx; i += 32) {
+            const size_t off = plane + (size_t)j * upitch + i;
+            const double ro = val(F_RO, off), tt = val(F_TT, off), rw = val(F_RW, off);
+            const double ri = 1.0 / ro;
+            const double u = val(F_RU, off) * ri, v = val(F_RV, off) * ri, w = rw * ri;
+            const double ke = u * u + v * v + w * w;
+            a[0] += ro;
+            a[1] += tt;
+            a[2] += 0.5 * ro * ke;
+            a[3] += 2.5 * ro * tt;
+            a[4] += -rw * (2.5 * (tt - t0) + 0.5 * ke);
+            a[6] += rw;
+            if (MAG) {
+                const double bx = val(F_BX, off), by = val(F_BY, off), bz = val(F_BZ, off);
+                a[5] += 0.5 * (bx * bx + by * by + bz * bz);
+            }
         }
+#pragma unroll
+    for (int q = 0; q < PROF_SUMS; ++q) {
+        for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+        if (lane == 0) red[warp][q] = a[q];
     }
-    const double cnt = (double)(float)n;   // FLOAT(NPX*NPY)
-    const double rom = block_sum(sro, red) / cnt;
-    const double ttm = block_sum(stt, red) / cnt;
-    const double kem = block_sum(ske, red) / cnt;
-    const double enm = block_sum(sen, red) / cnt;
-    const double mem = block_sum(sme, red) / cnt;
-    double sfc = 0.0;
-    for (int q = threadIdx.x; q < n; q += PROF_THREADS) {
-        const int i = q % npx, j = q / npx;
-        const size_t off = (size_t)K0 * uz + (size_t)(j + 1) * upitch + (i + 1);
-        const double ro = val(F_RO, off), tt = val(F_TT, off), rw = val(F_RW, off);
-        const double ri = 1.0 / ro;
-        const double u = val(F_RU, off) * ri, v = val(F_RV, off) * ri, w = rw * ri;
-        sfc += -rw * (2.5 * (tt - ttm) + 0.5 * (u * u + v * v + w * w));
-    }
-    const double fcm = block_sum(sfc, red) / cnt;
-    if (threadIdx.x == 0) {
-        out[MHD3D_PROF_RHO * npz + k] = rom;
-        out[MHD3D_PROF_T * npz + k] = ttm;
-        out[MHD3D_PROF_KE * npz + k] = kem;
-        out[MHD3D_PROF_ENTH * npz + k] = enm;
-        out[MHD3D_PROF_FCONV * npz + k] = fcm;
-        out[MHD3D_PROF_ME * npz + k] = mem;
+    __syncthreads();
+    if (threadIdx.x < PROF_SUMS) {
+        double x = 0.0;
+        for (int w = 0; w < PROF_WARPS; ++w) x += red[w][threadIdx.x];
+        part[((size_t)k * gridDim.y + blockIdx.y) * PROF_SUMS + threadIdx.x] = x;
     }
 }
 
-// FRADM from TTM (3dmhdsub.f:1663-1676): centred inside, one-sided at both walls
-__global__ void k_frad(double* __restrict__ out, const double* __restrict__ dzzdz, const double* __restrict__ rkapa,
-                       double hz, double repr, int npz)
+// A plane's means from its CTAs' sums, then FRADM from TTM
+// (3dmhdsub.f:1663-1676): centred inside, one-sided at both walls.  One CTA.
+template <bool F32>
+__global__ void k_profiles_fin(const void* __restrict__ ubuf, const double* __restrict__ bgd,
+                               const double* __restrict__ part, int split, double* __restrict__ out,
+                               const double* __restrict__ dzzdz, const double* __restrict__ rkapa, double hz,
+                               double repr, int npx, int npy, int npz, int upitch, size_t uz, size_t uf)
 {
+    const double cnt = (double)(float)(npx * npy);   // FLOAT(NPX*NPY)
+    for (int k = threadIdx.x; k < npz; k += blockDim.x) {
+        double a[PROF_SUMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int b = 0; b < split; ++b)
+#pragma unroll
+            for (int q = 0; q < PROF_SUMS; ++q) a[q] += part[((size_t)k * split + b) * PROF_SUMS + q];
+        const size_t t = (size_t)F_TT * uf + (size_t)(k + 1) * uz + upitch + 1;   // t0 of k_profiles
+        const double t0 = F32 ? bgd[bg_row(F_TT) * ((size_t)npz + 2) + k + 1]
+                                    + (double)reinterpret_cast<const float*>(ubuf)[t]
+                              : reinterpret_cast<const double*>(ubuf)[t];
+        const double ttm = a[1] / cnt;
+        out[MHD3D_PROF_RHO * npz + k] = a[0] / cnt;
+        out[MHD3D_PROF_T * npz + k] = ttm;
+        out[MHD3D_PROF_KE * npz + k] = a[2] / cnt;
+        out[MHD3D_PROF_ENTH * npz + k] = a[3] / cnt;
+        out[MHD3D_PROF_FCONV * npz + k] = (a[4] + 2.5 * (ttm - t0) * a[6]) / cnt;
+        out[MHD3D_PROF_ME * npz + k] = a[5] / cnt;
+    }
+    __syncthreads();
     const double* ttm = out + MHD3D_PROF_T * npz;   // ttm[k] is TTM(K=k+2)
     for (int k = threadIdx.x; k < npz; k += blockDim.x) {
         const int K = k + 2;
@@ -1745,15 +1753,25 @@ int profiles(Handle* h, double* out)
     if (!out) return MHD3D_ERR_ARG;
     if (int st = settle(h)) return st;
     const int npx = h->p.npx, npy = h->p.npy, npz = h->p.npz;
-    double* dout = h->stage;   // the staging field holds far more than MHD3D_NPROF x NPZ doubles
-    if (h->f32)
-        k_profiles<true><<<npz, PROF_THREADS, 0, h->st>>>(h->ubuf[h->cur], h->bgd, dout, npx, npy, npz, h->upitch,
-                                                         h->uz, h->uf, h->p.lmag);
-    else
-        k_profiles<false><<<npz, PROF_THREADS, 0, h->st>>>(h->ubuf[h->cur], h->bgd, dout, npx, npy, npz, h->upitch,
-                                                          h->uz, h->uf, h->p.lmag);
-    CK(cudaGetLastError());
-    k_frad<<<1, 256, 0, h->st>>>(dout, h->m.dzzdz, h->m.rkapa, h->p.hz, h->p.repr, npz);
+    // CTAs a plane: what the device holds at once, at most one per PROF_WARPS rows
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev);
+    const int rows = (npy + PROF_WARPS - 1) / PROF_WARPS, want = sms * PROF_CTAS / npz;
+    const int split = want < 1 ? 1 : (want < rows ? want : rows);
+    // the staging fields hold (npx+2)(npy+2) doubles a plane: at least 9, and 7 a CTA
+    double* const dout = h->stage;
+    double* const part = h->stage2;
+    auto run = [&](auto f32, auto mag) {
+        constexpr bool F = decltype(f32)::value;
+        k_profiles<F, decltype(mag)::value><<<dim3((unsigned)npz, (unsigned)split), 32 * PROF_WARPS, 0, h->st>>>(
+            h->ubuf[h->cur], h->bgd, part, npx, npy, npz, h->upitch, h->uz, h->uf);
+        k_profiles_fin<F><<<1, 256, 0, h->st>>>(h->ubuf[h->cur], h->bgd, part, split, dout, h->m.dzzdz, h->m.rkapa,
+                                                h->p.hz, h->p.repr, npx, npy, npz, h->upitch, h->uz, h->uf);
+    };
+    using Y = std::true_type;
+    using N = std::false_type;
+    if (h->f32) h->p.lmag ? run(Y{}, Y{}) : run(Y{}, N{});
+    else h->p.lmag ? run(N{}, Y{}) : run(N{}, N{});
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dout, sizeof(double) * MHD3D_NPROF * npz, cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));

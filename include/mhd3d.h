@@ -357,7 +357,9 @@ int mhd3d_conv3d_wgrad(int32_t cin, int32_t cout, const void* x, const void* dy,
  * means: 3*NPZ doubles of scratch).  mhd3d_closure_loss: adds the mean-square
  * error of pred [v][16] against target [v][12] to *loss and writes its
  * gradient dy [v][16] BF16.  mhd3d_adam: one Adam step on FP32 parameters
- * (step number t), optional BF16 copy.  mhd3d_closure_tendency: the
+ * (step number t), optional BF16 copy; mhd3d_adam_multi: the same step of
+ * count tensors (a host array), in one launch up to 16, as if one after the
+ * other (no two may overlap).  mhd3d_closure_tendency: the
  * tendencies of pred (16-byte aligned) for a handle's state, out[f][k][j][i]
  * (f = RU, RV, RW, TT, BX, BY, BZ); *flag set when the indicator trips.
  */
@@ -383,6 +385,16 @@ int mhd3d_closure_set_bias(void* handle, const float* bias);
 int mhd3d_coarsen(void* fine, int32_t fac, double* cstate, float* targets, void* stream);
 int mhd3d_closure_features(void* handle, const float* in_scale, void* feat, double* means, void* stream);
 int mhd3d_closure_loss(const float* pred, const float* target, int64_t nvox, void* dy, double* loss, void* stream);
+typedef struct {
+    float* p;
+    const float* g;
+    float* m;
+    float* v;
+    int64_t n;
+    void* p_bf16;   /* NULL: no copy */
+} mhd3d_adam_tensor;
+int mhd3d_adam_multi(const mhd3d_adam_tensor* tensors, int32_t count, float lr, float b1, float b2, float eps,
+                     int32_t t, void* stream);
 int mhd3d_adam(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2, float eps,
                int32_t t, void* p_bf16, void* stream);
 int mhd3d_closure_tendency(void* handle, const float* pred, const float* out_scale, float* out, int32_t* flag,

@@ -11,7 +11,7 @@ Every arithmetic step runs in the library (libmhd3d_gpu.so): coarsening and
 targets (mhd3d_coarsen), features, the tcgen05 convolutions and their input
 gradients (mhd3d_conv3d, mhd3d_conv3d_wtranspose), FP32 weight gradients
 (mhd3d_conv3d_wgrad_ws), the loss and its gradient (mhd3d_closure_loss), Adam
-(mhd3d_adam), the closure tendencies (mhd3d_closure_tendency) and, for
+(mhd3d_adam_multi), the closure tendencies (mhd3d_closure_tendency) and, for
 training on tendencies, their loss and adjoint (mhd3d_closure_tendency_loss,
 mhd3d_closure_tendency_adjoint).  torch provides device memory and streams.
 """
@@ -38,6 +38,12 @@ def _torch():
 def _check(st, what):
     if st:
         raise mhd3d.Mhd3dError(st, what)
+
+
+class _AdamTensor(C.Structure):
+    """mhd3d_adam_tensor"""
+    _fields_ = [("p", C.c_void_p), ("g", C.c_void_p), ("m", C.c_void_p), ("v", C.c_void_p), ("n", C.c_int64),
+                ("p_bf16", C.c_void_p)]
 
 
 class ClosureNet:
@@ -120,18 +126,17 @@ class ClosureNet:
         self.t = 0
 
     def zero_grad(self):
-        for g in self.dw + self.db:
-            g.zero_()
+        _torch()._foreach_zero_(self.dw + self.db)
 
     def adam_step(self, lr, stream, b1=0.9, b2=0.999, eps=1e-8):
         self.t += 1
-        for li in range(len(LAYERS)):
-            _check(self.lib.mhd3d_adam(_p(self.w[li]), _p(self.dw[li]), _p(self.m[li][0]), _p(self.v[li][0]),
-                                       self.w[li].numel(), lr, b1, b2, eps, self.t, _p(self.w16[li]),
-                                       C.c_void_p(stream)), "mhd3d_adam")
-            _check(self.lib.mhd3d_adam(_p(self.b[li]), _p(self.db[li]), _p(self.m[li][1]), _p(self.v[li][1]),
-                                       self.b[li].numel(), lr, b1, b2, eps, self.t, None, C.c_void_p(stream)),
-                   "mhd3d_adam")
+        rows = [(self.w[li], self.dw[li], self.m[li][0], self.v[li][0], self.w16[li]) for li in range(len(LAYERS))]
+        rows += [(self.b[li], self.db[li], self.m[li][1], self.v[li][1], None) for li in range(len(LAYERS))]
+        tensors = (_AdamTensor * len(rows))(*[
+            (p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), p.numel(), c.data_ptr() if c is not None else None)
+            for p, g, m, v, c in rows])
+        _check(self.lib.mhd3d_adam_multi(tensors, len(rows), lr, b1, b2, eps, self.t, C.c_void_p(stream)),
+               "mhd3d_adam_multi")
 
     def loss_and_grad(self, pred, target, stream):
         torch = _torch()

@@ -132,6 +132,7 @@ def gpu_lib() -> C.CDLL:
     lib.mhd3d_coarsen.argtypes = [vp, i32, vp, vp, vp]
     lib.mhd3d_closure_features.argtypes = [vp, vp, vp, vp, vp]
     lib.mhd3d_closure_loss.argtypes = [vp, vp, C.c_int64, vp, vp, vp]
+    lib.mhd3d_adam_multi.argtypes = [vp, i32, C.c_float, C.c_float, C.c_float, C.c_float, i32, vp]
     lib.mhd3d_adam.argtypes = [vp, vp, vp, vp, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_float, i32, vp, vp]
     lib.mhd3d_closure_tendency.argtypes = [vp, vp, vp, vp, vp, C.c_float, vp]
     lib.mhd3d_closure_tendency_loss.argtypes = [vp, vp, vp, C.c_int64, vp, vp, vp]

@@ -697,7 +697,9 @@ def main():
     peaks, peak_src = measured_peaks()
     launches = sum(stage_n)
     kernel_ms = sum(stage_ms) / max(launches, 1)
-    bytes_per_launch = 10 * nf * word * cells / 3.0
+    # words a cell and step: U in and out three times, Z out and in; the FMA build's stage 1
+    # writes no Z (9 nf), stage 2 reads the step's first state in its place
+    bytes_per_launch = (9 if args.mode == "fast" else 10) * nf * word * cells / 3.0
     achieved = bytes_per_launch / (kernel_ms / 1e3) / 1e9
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "stage_traffic.json")

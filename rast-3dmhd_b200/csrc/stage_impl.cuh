@@ -192,21 +192,23 @@ static cudaError_t launch_stage_t(int stage, const StageArgs& a, cudaStream_t st
 {
     const int nty = (a.s.npy + TY - 1) / TY;
     dim3 grid(a.ntx * nty, a.nchunks);
-    switch (stage) {
-#define L_(S)                                                                                              \
+#define L_(S, ...)                                                                                         \
     case S: {                                                                                              \
         constexpr size_t smem = Lay<MAG, S>::BYTES;                                                        \
         static std::atomic<unsigned long long> attr_set{0};                                                \
-        cudaError_t ae = smem_attr_once(attr_set, reinterpret_cast<const void*>(k_stage<MAG, ROT, S>), smem); \
+        cudaError_t ae = smem_attr_once(attr_set, reinterpret_cast<const void*>(k_stage<MAG, ROT, __VA_ARGS__>), smem); \
         if (ae != cudaSuccess) return ae;                                                                  \
-        return launch_chained(k_stage<MAG, ROT, S>, grid, NT, smem, st, a);                                      \
+        return launch_chained(k_stage<MAG, ROT, __VA_ARGS__>, grid, NT, smem, st, a);                      \
     }
-        L_(0) L_(1) L_(2) L_(3)
-#undef L_
+#if MHD3D_FAST_BODY
+    if (a.z_stored) switch (stage) { L_(1, 1, true) L_(2, 2, true) }
+#endif
+    switch (stage) {
+        L_(0, 0) L_(1, 1) L_(2, 2) L_(3, 3)
     default:
         return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
+#undef L_
 }
 
 cudaError_t launch_stage(int stage, const StageArgs& a, cudaStream_t st)

@@ -5,7 +5,10 @@
 // state U0 the step began with, which is still in the buffer stage 2 writes
 // (a cell is read by the thread that then overwrites it, and by no other).
 // That is 64 of the 640 bytes a cell and step, and one rounding less: errors
-// against 80-bit arithmetic fall by 13-15 % in every field.
+// against 80-bit arithmetic fall by 13-15 % in every field.  U1-U0 carries the
+// rounding of U1, which ZETA1/GAM1 scales: a scheme with |ZETA1| > |GAM1| (the
+// reference's ratio is -0.53) would lose by it, up to GAM1 = 0, where U1 holds
+// no F1 at all, so it has Z stored (ZST; StageArgs.z_stored).
 //
 // Bound by DRAM traffic in flight (12 warps an SM, two planes in the ring
 // beyond the two in use, three in stage 1) together with the latency of a
@@ -53,8 +56,8 @@ struct Lay {
 };
 
 // STAGE 0: right-hand side only (written to f_out); STAGE 1..3: the RK3
-// substeps of STEP (3dmhdsub.f:874-1169).
-template <bool MAG, bool ROT, int STAGE>
+// substeps of STEP (3dmhdsub.f:874-1169).  ZST: stage 1 stores Z, stage 2 reads it.
+template <bool MAG, bool ROT, int STAGE, bool ZST = false>
 __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant__ StageArgs a)
 {
     using L = Lay<MAG, STAGE>;
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
     grid_wait();   // what follows reads what the kernels before wrote
     const double DT = ctl->dt;
     const double cu = STAGE == 1 ? s.gam1 * DT : STAGE == 2 ? s.gam2 * DT : s.gam3 * DT;
-    const double cz = s.zeta2 * DT;
+    const double cz = (STAGE == 1 ? s.zeta1 : s.zeta2) * DT;
     const double C13 = s.c13, C23 = s.c23, C43 = s.c43;
     MarchCol col;
     {
@@ -153,7 +156,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
         fence_proxy_async();
         mbar_expect_tx(&bars[NR + zs], z_bytes);
         // stage 2: the state the step began with, still in the output buffer
-        if (STAGE == 2) tma_load4(sz + (size_t)zs * L::ZT, &a.map_o, &bars[NR + zs], x0 + UOFS + 1, y0 + 1, k + 1, 0);
+        if (STAGE == 2 && !ZST) tma_load4(sz + (size_t)zs * L::ZT, &a.map_o, &bars[NR + zs], x0 + UOFS + 1, y0 + 1, k + 1, 0);
         else tma_load4(sz + (size_t)zs * L::ZT, &a.map_z, &bars[NR + zs], x0, y0, k, 0);
         z_hi = k;
     };
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                                 zby = zt_[F_BY * NT];
                                 zbz = zt_[F_BZ * NT];
                             }
-                            if (STAGE == 2) {
+                            if (STAGE == 2 && !ZST) {
                                 // Z = U1 + ZETA1*DT*F1 with GAM1*DT*F1 = U1 - U0
                                 zu = fma(s.zr10, c.ru - zu, c.ru);
                                 zv = fma(s.zr10, c.rv - zv, c.rv);
@@ -265,9 +268,9 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                                               {nr, nbx, nby, nu, nv, nw, nt, nbz});
                             else
                                 store_cell<5>(pl, a.uf, ucol, hc, {F_RO, F_RU, F_RV, F_RW, F_TT}, {nr, nu, nv, nw, nt});
-                            // Z for stage 3: Z = U + ZETA*DT*F; on the walls only
+                            // Z for the next stage: Z = U + ZETA*DT*F; on the walls only
                             // RO, BX, BY are ever read back
-                            if (STAGE == 2) {
+                            if (STAGE == 2 || ZST) {
                                 double* zo = a.z + zc;
                                 zo[F_RO * a.zf] = nr + cz * c.fr;
                                 if (MAG) {

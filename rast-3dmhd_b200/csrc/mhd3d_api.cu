@@ -61,7 +61,7 @@ struct Handle {
     PlaneBg* pb = nullptr;        // per interior plane
     PlaneZ* pz = nullptr;         // per U plane (FP64)
     MarchRun run{};
-    bool z_stored = false;        // StageArgs.z_stored
+    bool general = false;         // StageArgs.general
     std::vector<double> faz_h, fbz_h, fcz_h;   // host copies of the z stencil factors
     std::vector<double> rka_h, dka_h, ddz_h;   // and of RKAPA, DKAPA, DDZ
     ColC* cxy = nullptr;                       // FP32 column constants: NX in x, then NY in y
@@ -939,7 +939,7 @@ StageArgs make_args(Handle* h)
     a.s = h->s;
     a.pz = h->pz;
     a.run = h->run;
-    a.z_stored = h->z_stored;
+    a.general = h->general;
     a.uf = h->uf;
     a.uz = h->uz;
     a.zf = h->zf;
@@ -1361,8 +1361,9 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
     s.c13 = p->c13; s.c23 = p->c23; s.c43 = p->c43;
     s.hx = p->hx; s.h2x = p->h2x; s.hy = p->hy; s.h2y = p->h2y; s.hz = p->hz; s.h2z = p->h2z;
     s.gam1 = p->gam1; s.gam2 = p->gam2; s.gam3 = p->gam3; s.zeta1 = p->zeta1; s.zeta2 = p->zeta2;
-    h->z_stored = !(std::fabs(p->zeta1) <= std::fabs(p->gam1)) || p->gam1 == 0.0;
-    s.zr10 = h->z_stored ? 0.0 : p->zeta1 / p->gam1;
+    s.wallz = (p->lmag && p->ibcon != 0) || p->itcon == 3;
+    h->general = !(std::fabs(p->zeta1) <= std::fabs(p->gam1)) || p->gam1 == 0.0 || s.wallz;
+    s.zr10 = h->general ? 0.0 : p->zeta1 / p->gam1;
     s.cv = p->cv; s.ocv = p->ocv; s.ore = p->ore; s.re = p->re; s.repr = p->repr;
     s.theta = p->theta; s.grav = p->grav; s.gamma = p->gamma; s.ogamma = 1.0 / p->gamma; s.sf = p->sf;
     s.rm = p->rm; s.omx = p->omx; s.omz = p->omz; s.orm = p->orm; s.obeta = p->obeta;

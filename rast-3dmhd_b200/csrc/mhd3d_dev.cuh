@@ -53,7 +53,7 @@ struct Scalars {
     double c13, c23, c43;
     double hx, h2x, hy, h2y, hz, h2z;
     double gam1, gam2, gam3, zeta1, zeta2;
-    double zr10;       // ZETA1/GAM1 (FMA build, unless z_stored)
+    double zr10;       // ZETA1/GAM1 (FMA build, but for its GEN instances)
     double cv, ocv, ore, re, repr, theta, grav, gamma, ogamma, sf, rm;
     double omx, omz, orm, obeta;
     double tmp_cond;   // OCV/REPR          (3dmhdsub.f:1584)
@@ -70,6 +70,7 @@ struct Scalars {
     float ogamma_f, gamma_f, obeta_f;   // 1/GAMMA, GAMMA, OBETA rounded to FP32 (fast-mode CFL screening)
     int npx, npy, npz, pitch;
     int lmag, lrot, izcon, itcon, ibcon, plume;
+    int wallz;         // BCON leaves a wall value to the RK3 update: BZ (IBC not 0), TT on the top wall (ITC=3)
 };
 
 // Step bookkeeping kept on the device so that many steps run without a
@@ -127,7 +128,7 @@ struct StageArgs {
     CUtensorMap map_o;      // tiles without halo of the output U buffer (stage 2 of the FMA build)
     const double* u_in;     // current state
     double* u_out;          // next state (other ping-pong buffer)
-    double* z;              // Z (reference rounding: read in stages 2,3; written in stages 1,2; FMA build: see z_stored)
+    double* z;              // Z (reference rounding: read in stages 2,3; written in stages 1,2; FMA build: see stage_march.cuh)
     double* f_out;          // RHS output (RHS-only launch), Z layout
     Control* ctl;
     Accum* acc;
@@ -141,7 +142,7 @@ struct StageArgs {
     int ntx;                // tiles along x
     int nchunks;            // z chunks (chunk_start)
     int end_step;           // the last CTA of stage 3 ends the step (finalize.cuh)
-    int z_stored;           // FMA build: Z of stage 2 is stored by stage 1 (|ZETA1| > |GAM1|), not formed from U1 and U0
+    int general;            // FMA build: the GEN instances (stage_march.cuh), where |ZETA1| > |GAM1| or wallz
     unsigned long long w4key;
     long long wait_first;   // poll limit of a CTA's first ring wait (WAIT_LIMIT; lowered only by tests)
 };

@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                     else
                         store_cell<5>(pl, a.uf, ucol, hc, {F_RO, F_RU, F_RV, F_RW, F_TT}, {nr, nu, nv, nw, nt});
                     // ---- Z for the next stage: Z = U + ZETA*DT*F (loops 190-260, 390-460).
-                    //      On the walls only RO, BX, BY are ever read back.
+                    //      On the walls only RO, BX, BY, and what else BCON does not rewrite (wallz).
                     if (STAGE < 3) {
                         double* zo = a.z + zc;
                         zo[F_RO * a.zf] = nr + cz * fr;
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                             zo[F_BX * a.zf] = nbx + cz * w1;
                             zo[F_BY * a.zf] = nby + cz * w2;
                         }
-                        if (!wall) {
+                        if (!wall || s.wallz) {
                             zo[F_RU * a.zf] = nu + cz * fu;
                             zo[F_RV * a.zf] = nv + cz * fv;
                             zo[F_RW * a.zf] = nw + cz * fw;

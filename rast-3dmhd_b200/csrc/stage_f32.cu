@@ -489,14 +489,14 @@ __device__ __forceinline__ void stage32_item(const StageArgs32& a, const int til
                                              {nr, nbx, nby, nu, nv, nw, nt, nbz});
                     else
                         store_cell<5, float>(pl, a.uf, ucol, hc, {F_RO, F_RU, F_RV, F_RW, F_TT}, {nr, nu, nv, nw, nt});
-                    if (STAGE < 3) {
+                    if (STAGE < 3) {   // Z; on the walls only RO, BX, BY, and what else BCON does not rewrite (wallz)
                         float* zo = a.z + zc;
                         zo[F_RO * a.zf] = nr + cz * fr;
                         if (MAG) {
                             zo[F_BX * a.zf] = nbx + cz * w1;
                             zo[F_BY * a.zf] = nby + cz * w2;
                         }
-                        if (!wall) {
+                        if (!wall || s.wallz) {
                             zo[F_RU * a.zf] = nu + cz * fu;
                             zo[F_RV * a.zf] = nv + cz * fv;
                             zo[F_RW * a.zf] = nw + cz * fw;

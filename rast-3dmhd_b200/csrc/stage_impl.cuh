@@ -201,7 +201,7 @@ static cudaError_t launch_stage_t(int stage, const StageArgs& a, cudaStream_t st
         return launch_chained(k_stage<MAG, ROT, __VA_ARGS__>, grid, NT, smem, st, a);                      \
     }
 #if MHD3D_FAST_BODY
-    if (a.z_stored) switch (stage) { L_(1, 1, true) L_(2, 2, true) }
+    if (a.general) switch (stage) { L_(1, 1, true) L_(2, 2, true) L_(3, 3, true) }
 #endif
     switch (stage) {
         L_(0, 0) L_(1, 1) L_(2, 2) L_(3, 3)

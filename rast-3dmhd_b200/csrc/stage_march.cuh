@@ -8,7 +8,11 @@
 // against 80-bit arithmetic fall by 13-15 % in every field.  U1-U0 carries the
 // rounding of U1, which ZETA1/GAM1 scales: a scheme with |ZETA1| > |GAM1| (the
 // reference's ratio is -0.53) would lose by it, up to GAM1 = 0, where U1 holds
-// no F1 at all, so it has Z stored (ZST; StageArgs.z_stored).
+// no F1 at all, so it has Z stored by stage 1.
+//
+// GEN instances (StageArgs.general) are for what the others leave out to stay
+// as fast as they are: Z stored by stage 1, and wall values that BCON does not
+// rewrite (BZ with IBC not 0, TT on the top wall with ITC=3).
 //
 // Bound by DRAM traffic in flight (12 warps an SM, two planes in the ring
 // beyond the two in use, three in stage 1) together with the latency of a
@@ -56,8 +60,8 @@ struct Lay {
 };
 
 // STAGE 0: right-hand side only (written to f_out); STAGE 1..3: the RK3
-// substeps of STEP (3dmhdsub.f:874-1169).  ZST: stage 1 stores Z, stage 2 reads it.
-template <bool MAG, bool ROT, int STAGE, bool ZST = false>
+// substeps of STEP (3dmhdsub.f:874-1169).
+template <bool MAG, bool ROT, int STAGE, bool GEN = false>
 __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant__ StageArgs a)
 {
     using L = Lay<MAG, STAGE>;
@@ -156,7 +160,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
         fence_proxy_async();
         mbar_expect_tx(&bars[NR + zs], z_bytes);
         // stage 2: the state the step began with, still in the output buffer
-        if (STAGE == 2 && !ZST) tma_load4(sz + (size_t)zs * L::ZT, &a.map_o, &bars[NR + zs], x0 + UOFS + 1, y0 + 1, k + 1, 0);
+        if (STAGE == 2 && !GEN) tma_load4(sz + (size_t)zs * L::ZT, &a.map_o, &bars[NR + zs], x0 + UOFS + 1, y0 + 1, k + 1, 0);
         else tma_load4(sz + (size_t)zs * L::ZT, &a.map_z, &bars[NR + zs], x0, y0, k, 0);
         z_hi = k;
     };
@@ -212,6 +216,13 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                     const size_t zc = (size_t)k * a.zz + zcol;
                     if (STAGE != 0 && bot)
                         store_cell<1>(a.u_out + (size_t)(npz + 1) * a.uz, a.uf, ucol, hc, {F_RO}, {ghost});
+                    if (GEN && top) {
+                        // FT's dw/dz is central on the wall, with the ghost plane
+                        const double* g = a.u_in + ucol;
+                        const double wz = (c.nw - g[F_RW * a.uf] * (1.0 / g[F_RO * a.uf])) * zk.az;
+                        c.ft += c.ri * run.tmpa * run.c43 * (wz * (wz - c.s) - c.wz * (c.wz - c.s))
+                              - run.ocv * c.tt * (wz - c.wz);
+                    }
                     if (STAGE == 0) {
                         a.f_out[zc + 0 * a.zf] = wall ? 0.0 : c.fu;
                         a.f_out[zc + 1 * a.zf] = wall ? 0.0 : c.fv;
@@ -242,7 +253,7 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                                 zby = zt_[F_BY * NT];
                                 zbz = zt_[F_BZ * NT];
                             }
-                            if (STAGE == 2 && !ZST) {
+                            if (STAGE == 2 && !GEN) {
                                 // Z = U1 + ZETA1*DT*F1 with GAM1*DT*F1 = U1 - U0
                                 zu = fma(s.zr10, c.ru - zu, c.ru);
                                 zv = fma(s.zr10, c.rv - zv, c.rv);
@@ -268,16 +279,16 @@ __global__ void __launch_bounds__(NT, MHD3D_MINB) k_stage(const __grid_constant_
                                               {nr, nbx, nby, nu, nv, nw, nt, nbz});
                             else
                                 store_cell<5>(pl, a.uf, ucol, hc, {F_RO, F_RU, F_RV, F_RW, F_TT}, {nr, nu, nv, nw, nt});
-                            // Z for the next stage: Z = U + ZETA*DT*F; on the walls only
-                            // RO, BX, BY are ever read back
-                            if (STAGE == 2 || ZST) {
+                            // Z for the next stage: Z = U + ZETA*DT*F; on the walls only RO, BX,
+                            // BY, and what else BCON does not rewrite (GEN)
+                            if (STAGE == 2 || (STAGE == 1 && GEN)) {
                                 double* zo = a.z + zc;
                                 zo[F_RO * a.zf] = nr + cz * c.fr;
                                 if (MAG) {
                                     zo[F_BX * a.zf] = nbx + cz * c.w1;
                                     zo[F_BY * a.zf] = nby + cz * c.w2;
                                 }
-                                if (!wall) {
+                                if (!wall || GEN) {
                                     zo[F_RU * a.zf] = nu + cz * c.fu;
                                     zo[F_RV * a.zf] = nv + cz * c.fv;
                                     zo[F_RW * a.zf] = nw + cz * c.fw;

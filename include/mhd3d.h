@@ -162,7 +162,8 @@ int mhd3d_step(void* handle, int32_t nsteps,
  * Only interior cells (I=2..NX-1, J=2..NY-1, K=2..NZ-1) are written.
  * Values on the wall planes that BCON overwrites (FU,FV,FW,FT and WW3 at
  * K=2 and K=NZ-1) are written as 0; the reference computes them from the
- * ghost planes and then discards them.
+ * ghost planes and then discards them.  When a bounded wait gives up
+ * (MHD3D_ERR_TIMEOUT) nothing is written, and later steps are not affected.
  */
 int mhd3d_fluxes(void* handle,
                  double* fu, double* fv, double* fw, double* fr, double* ft,

@@ -1753,13 +1753,25 @@ int fluxes(Handle* h, double* const out[8])
 {
     CK(cudaSetDevice(h->dev));
     if (int st = settle(h)) return st;
-    if (!h->fout) CK(cudaMalloc(&h->fout, (h->f32 ? sizeof(float) : sizeof(double)) * h->nf * h->zf));
+    // the launch reports a wait that gave up in a Control of its own, behind
+    // the right-hand sides: it is no step, and stops none
+    const size_t bytes = (h->f32 ? sizeof(float) : sizeof(double)) * h->nf * h->zf;
+    if (!h->fout) CK(cudaMalloc(&h->fout, bytes + sizeof(Control)));
+    Control* const ctl = reinterpret_cast<Control*>(reinterpret_cast<char*>(h->fout) + bytes);
+    CK(cudaMemsetAsync(ctl, 0, sizeof(Control), h->st));
     if (h->f32) {
-        CK(f32::launch_stage(0, make_args32(h), h->st));
+        StageArgs32 a = make_args32(h);
+        a.ctl = ctl;
+        CK(f32::launch_stage(0, a, h->st));
     } else {
         StageArgs a = make_args(h);
+        a.ctl = ctl;
         CK(launch_stage(h, 0, a));
     }
+    Control c{};
+    CK(cudaMemcpyAsync(&c, ctl, sizeof(Control), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaStreamSynchronize(h->st));
+    if (c.stop) return c.status;
     const int npx = h->p.npx, npy = h->p.npy, npz = h->p.npz;
     const size_t nfort = (size_t)(npx + 2) * (npy + 2) * (npz + 2);
     for (int fi = 0; fi < h->nf; ++fi) {

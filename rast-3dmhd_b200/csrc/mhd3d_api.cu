@@ -1672,14 +1672,18 @@ int step_async(Handle* h, int n)
     if (n < 0) return MHD3D_ERR_ARG;
     // a call that starts from a synced state clears the stop flag, where the
     // last sync saw it; DT of the current state comes from the last stage-3
-    // reduction, or from a fresh CFL pass after the state changed
+    // reduction, or from a fresh CFL pass after the state changed.  Captured
+    // steps always hold the reset: a replay starts from a synced state too,
+    // and nothing is known here of the stops before it
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(h->st, &cap));
     if (!h->dt_valid) {
         int st = initial_dt(h);
         if (st) return st;
-    } else if (h->pending == 0 && h->need_reset) {
+    } else if (h->pending == 0 && (h->need_reset || cap != cudaStreamCaptureStatusNone)) {
         k_reset<<<1, 1, 0, h->st>>>(h->ctl, h->acc, 1, h->w4key);
         CK(cudaGetLastError());
-        h->need_reset = false;
+        h->need_reset = cap != cudaStreamCaptureStatusNone;   // a capture has not run yet
     }
     int cur = h->cur_base ^ (h->pending & 1);
     for (int s = 0; s < n; ++s) {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -100,6 +101,7 @@ struct Handle {
         if (e_ != cudaSuccess) {                                                                 \
             std::fprintf(stderr, "mhd3d: %s failed: %s (%s:%d)\n", #x, cudaGetErrorString(e_),   \
                          __FILE__, __LINE__);                                                     \
+            (void)cudaGetLastError();   /* reported here, not again by the next call */           \
             return e_ == cudaErrorMemoryAllocation ? MHD3D_ERR_NOMEM : MHD3D_ERR_CUDA;            \
         }                                                                                        \
     } while (0)
@@ -1504,9 +1506,32 @@ int set_background(Handle* h)
     return MHD3D_OK;
 }
 
+// Whether `bytes` from device address p lie inside one allocation
+bool in_allocation(const void* p, size_t bytes)
+{
+    typedef CUresult (*RangeFn)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static std::atomic<RangeFn> range{nullptr};
+    RangeFn f = range.load();
+    if (!f) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        f = reinterpret_cast<RangeFn>(fn);
+        range.store(f);
+    }
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr a = reinterpret_cast<CUdeviceptr>(p);
+    return f(&base, &size, a) == CUDA_SUCCESS && a - base <= size && bytes <= size - (a - base);
+}
+
 // Whether the field arrays can be read or written by kernels in place: memory
-// of the handle's device, on 8 bytes, no two arrays overlapping (a copy through
-// the staging fields takes them in order).
+// of the handle's device, on 8 bytes, each inside one allocation (an array that
+// ends too soon is left to the copy, which refuses it), no two arrays
+// overlapping (a copy through the staging fields takes them in order).
 bool in_place(const Handle* h, const void* const f[8], size_t bytes)
 {
     for (int i = 0; i < h->nf; ++i) {
@@ -1516,7 +1541,9 @@ bool in_place(const Handle* h, const void* const f[8], size_t bytes)
             (void)cudaGetLastError();
             return false;
         }
-        if (at.type != cudaMemoryTypeDevice || at.device != h->dev || (reinterpret_cast<uintptr_t>(f[i]) & 7u)) return false;
+        if (at.type != cudaMemoryTypeDevice || at.device != h->dev || (reinterpret_cast<uintptr_t>(f[i]) & 7u) ||
+            !in_allocation(f[i], bytes))
+            return false;
         for (int j = 0; j < i; ++j) {
             const char *x = static_cast<const char*>(f[i]), *y = static_cast<const char*>(f[j]);
             if (y && x < y + bytes && y < x + bytes) return false;

@@ -40,7 +40,7 @@ namespace MHD3D_NS {
 #endif
 // raw-plane ring slots
 constexpr int NRAW = MHD3D_NRAW;
-static_assert(NRAW >= 3 && NRAW <= 6, "three to six ring slots (NRAW+2 mbarriers)");
+static_assert(NRAW >= 3 && NRAW <= 6, "three to six ring slots");
 
 // store a cell of U and the periodic halo copies COMMUNICATE would make of it
 __device__ __forceinline__ void store_u(double* __restrict__ u, size_t fofs, const StageArgs& a, int gi, int gj,

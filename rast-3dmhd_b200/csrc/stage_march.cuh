@@ -53,7 +53,7 @@ struct Lay {
     static constexpr int RI_OFF = NR * RAW_SLOT;
     static constexpr int Z_OFF = ((RI_OFF + 2 * BSLOT) * 8 + 127) / 128 * 128 / 8;
     static constexpr int BAR_OFF = Z_OFF + (STAGE >= 2 ? NZS : 0) * ZT;
-    static constexpr int RED_OFF = BAR_OFF + 8;
+    static constexpr int RED_OFF = BAR_OFF + (NR + NZS + 1) / 2 * 2;   // an mbarrier a slot
     static constexpr int FLAG_OFF = RED_OFF + (NT / 32) * 8;
     static constexpr int TOTAL = FLAG_OFF + 2;
     static constexpr size_t BYTES = (size_t)TOTAL * 8 + 128;

@@ -12,7 +12,7 @@ reference checkout.
 
 The checkout's location comes from --src, else the environment variable
 MHD3D_REFERENCE_SRC, else the container's read-only mount.  With
---if-present missing sources are not an error.
+--if-present sources that are missing altogether are not an error.
 """
 from __future__ import annotations
 
@@ -56,6 +56,6 @@ if __name__ == "__main__":
     ap.add_argument("--if-present", action="store_true",
                     help="exit quietly when the reference sources are absent")
     a = ap.parse_args()
-    if a.if_present and not all(os.path.exists(os.path.join(a.src, f)) for f in ("3dmhdsub.f", "3dmhdparam.f")):
+    if a.if_present and not any(os.path.exists(os.path.join(a.src, f)) for f in ("3dmhdsub.f", "3dmhdparam.f")):
         sys.exit(0)
     print(build(a.src, a.out))

@@ -35,7 +35,7 @@ struct Handle {
     int cur = 0;               // ubuf[cur] holds the current state
     CUtensorMap map_u[2];      // TMA maps of the two U buffers
     CUtensorMap map_z;
-    CUtensorMap map_o[2];      // tiles without halo of the two U buffers
+    CUtensorMap map_o[2];      // tiles without halo of the two U buffers (FP64)
     CUtensorMap emap_u[2];     // the same for the tile rows of an ensemble (FP32 members)
     CUtensorMap emap_z;
     int ety = 0;               // tile rows emap_* were made for (0: none)
@@ -1162,8 +1162,9 @@ int create(const mhd3d_params* p, const double* const arrs[14], void** out)
         for (int b = 0; b < 2; ++b) {
             int st2 = make_map(&h->map_u[b], h->ualloc[b], du, bu, h->f32);
             if (st2) return st2;
+            if (h->f32) continue;
             const cuuint32_t bo[4] = {TX, (cuuint32_t)ty, 1, (cuuint32_t)h->nf};
-            st2 = make_map(&h->map_o[b], h->ualloc[b], du, bo, h->f32);
+            st2 = make_map(&h->map_o[b], h->ualloc[b], du, bo);
             if (st2) return st2;
         }
         const cuuint64_t dz[4] = {(cuuint64_t)h->zpitch, (cuuint64_t)h->zrows, (cuuint64_t)npz, (cuuint64_t)h->nf};
@@ -2080,16 +2081,12 @@ int ens_set_tile(Ensemble* e, int ty)
     return ens_layout(e);
 }
 
-// set every member's z chunk length (<= 0: the single-grid default) and re-lay the work table
+// set every member's z chunk length (planes, at least three) and re-lay the work table
 int ens_set_zlen(Ensemble* e, int zlen)
 {
     for (Handle* h : e->mem) {
         const int npz = h->p.npz;
-        int nch;
-        if (zlen > 0) nch = std::max(1, npz / std::max(zlen, 3));
-        else nch = (npz + 63) / 64;
-        while (nch > 1 && npz / nch < 3) --nch;
-        h->nchunks = nch;
+        h->nchunks = std::max(1, npz / std::max(zlen, 3));
     }
     return ens_layout(e);
 }
@@ -2284,7 +2281,8 @@ int ens_tune(Ensemble* e, int steps, int32_t* zlen_out, int32_t* ctas_out, doubl
     if (st2) return st2;
     e->ctas_per_sm = best_c;
     if (int s3 = ens_set_tile(e, best_t)) return s3;
-    if (int s3 = ens_set_zlen(e, best_z)) return s3;
+    if (best_z)
+        if (int s3 = ens_set_zlen(e, best_z)) return s3;
     if (zlen_out) *zlen_out = best_z;
     if (ctas_out) *ctas_out = best_c;
     if (ms_out) *ms_out = best;

@@ -267,19 +267,24 @@ __global__ void k_pack_interior32(const float* __restrict__ f, double* __restric
 // are FP64, in a fixed order.  Bound by the read of the state: a plane's rows
 // are shared by enough CTAs to fill the device, and every field is read once.
 // FCONV needs the deviations from the plane's mean temperature, known only at
-// the end: the sums take them from the plane's first cell (as small), and
-// the mean of RW corrects for the difference.
+// the end: the sums take them from the mean of a sample of the plane's cells
+// (about as small), and the mean of RW corrects for the difference.  The
+// plane's first cell in the sample's place made the error 20 to 40 times that
+// of the two-pass form where that cell lies far from the mean (11 times the
+// temperature around it); with the sample it is as large as that form's.  A
+// sample of 256 cells was no closer and took 3 to 11 us more.
 // A call on 256x256x128, host and copy included: FP64 143 us, FP32 130; one
 // CTA a plane with a second pass for FCONV took 585 and 744.  3 CTAs an SM
 // (no spills) 177 and 152.
 constexpr int PROF_WARPS = 8, PROF_SUMS = 7, PROF_CTAS = 4;
+constexpr int PROF_PART = PROF_SUMS + 1;   // a CTA's sums, and the sample's mean
 
 template <bool F32, bool MAG>
 __global__ void __launch_bounds__(32 * PROF_WARPS, PROF_CTAS)
 k_profiles(const void* __restrict__ ubuf, const double* __restrict__ bgd, double* __restrict__ part, int npx, int npy,
            int npz, int upitch, size_t uz, size_t uf)
 {
-    __shared__ double red[PROF_WARPS][PROF_SUMS];
+    __shared__ double red[PROF_WARPS][PROF_SUMS], smp;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x;   // interior plane, Fortran K = k+2
     const int K0 = k + 1;       // U plane index
@@ -293,7 +298,15 @@ k_profiles(const void* __restrict__ ubuf, const double* __restrict__ bgd, double
         return reinterpret_cast<const double*>(ubuf)[(size_t)f * uf + off];
     };
     const size_t plane = (size_t)K0 * uz + upitch + 1;
-    const double t0 = val(F_TT, plane);
+    // 32 cells, in rows and columns of their own, the same in every CTA
+    if (warp == 0) {
+        const int j = (int)((2ll * lane + 1) * npy / 64), i = (int)((2ll * ((13 * lane + 7) & 31) + 1) * npx / 64);
+        double t = val(F_TT, plane + (size_t)j * upitch + i);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) smp = t * (1.0 / 32);
+    }
+    __syncthreads();
+    const double t0 = smp;
     double a[PROF_SUMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // RO, TT, KE, enthalpy, FCONV, ME, RW
     for (int j = blockIdx.y * PROF_WARPS + warp; j < npy; j += gridDim.y * PROF_WARPS)
         for (int i = lane; i < npx; i += 32) {
@@ -322,28 +335,25 @@ k_profiles(const void* __restrict__ ubuf, const double* __restrict__ bgd, double
     if (threadIdx.x < PROF_SUMS) {
         double x = 0.0;
         for (int w = 0; w < PROF_WARPS; ++w) x += red[w][threadIdx.x];
-        part[((size_t)k * gridDim.y + blockIdx.y) * PROF_SUMS + threadIdx.x] = x;
+        part[((size_t)k * gridDim.y + blockIdx.y) * PROF_PART + threadIdx.x] = x;
+    } else if (threadIdx.x == PROF_SUMS) {
+        part[((size_t)k * gridDim.y + blockIdx.y) * PROF_PART + PROF_SUMS] = t0;
     }
 }
 
 // A plane's means from its CTAs' sums, then FRADM from TTM
 // (3dmhdsub.f:1663-1676): centred inside, one-sided at both walls.  One CTA.
-template <bool F32>
-__global__ void k_profiles_fin(const void* __restrict__ ubuf, const double* __restrict__ bgd,
-                               const double* __restrict__ part, int split, double* __restrict__ out,
+__global__ void k_profiles_fin(const double* __restrict__ part, int split, double* __restrict__ out,
                                const double* __restrict__ dzzdz, const double* __restrict__ rkapa, double hz,
-                               double repr, int npx, int npy, int npz, int upitch, size_t uz, size_t uf)
+                               double repr, int npx, int npy, int npz)
 {
     const double cnt = (double)(float)(npx * npy);   // FLOAT(NPX*NPY)
     for (int k = threadIdx.x; k < npz; k += blockDim.x) {
         double a[PROF_SUMS] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         for (int b = 0; b < split; ++b)
 #pragma unroll
-            for (int q = 0; q < PROF_SUMS; ++q) a[q] += part[((size_t)k * split + b) * PROF_SUMS + q];
-        const size_t t = (size_t)F_TT * uf + (size_t)(k + 1) * uz + upitch + 1;   // t0 of k_profiles
-        const double t0 = F32 ? bgd[bg_row(F_TT) * ((size_t)npz + 2) + k + 1]
-                                    + (double)reinterpret_cast<const float*>(ubuf)[t]
-                              : reinterpret_cast<const double*>(ubuf)[t];
+            for (int q = 0; q < PROF_SUMS; ++q) a[q] += part[((size_t)k * split + b) * PROF_PART + q];
+        const double t0 = part[(size_t)k * split * PROF_PART + PROF_SUMS];
         const double ttm = a[1] / cnt;
         out[MHD3D_PROF_RHO * npz + k] = a[0] / cnt;
         out[MHD3D_PROF_T * npz + k] = ttm;
@@ -1832,15 +1842,15 @@ int profiles(Handle* h, double* out)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev);
     const int rows = (npy + PROF_WARPS - 1) / PROF_WARPS, want = sms * PROF_CTAS / npz;
     const int split = want < 1 ? 1 : (want < rows ? want : rows);
-    // the staging fields hold (npx+2)(npy+2) doubles a plane: at least 9, and 7 a CTA
+    // the staging fields hold (npx+2)(npy+2) doubles a plane: at least 16, and 8 a CTA
     double* const dout = h->stage;
     double* const part = h->stage2;
     auto run = [&](auto f32, auto mag) {
         constexpr bool F = decltype(f32)::value;
         k_profiles<F, decltype(mag)::value><<<dim3((unsigned)npz, (unsigned)split), 32 * PROF_WARPS, 0, h->st>>>(
             h->ubuf[h->cur], h->bgd, part, npx, npy, npz, h->upitch, h->uz, h->uf);
-        k_profiles_fin<F><<<1, 256, 0, h->st>>>(h->ubuf[h->cur], h->bgd, part, split, dout, h->m.dzzdz, h->m.rkapa,
-                                                h->p.hz, h->p.repr, npx, npy, npz, h->upitch, h->uz, h->uf);
+        k_profiles_fin<<<1, 256, 0, h->st>>>(part, split, dout, h->m.dzzdz, h->m.rkapa, h->p.hz, h->p.repr, npx, npy,
+                                             npz);
     };
     using Y = std::true_type;
     using N = std::false_type;

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
             if (lane == 0) mbar_arrive(accempty);
             if (!emit) return true;
             const int m = warp * 32 + lane;
-            const bool own = x0 + m < nx;   // for nx < 128 the tile repeats the row's period
+            const bool own = x0 + m < nx;   // lanes beyond the row's end store nothing
             const size_t vox = ((size_t)zz * ny + yo) * nx + (own ? x0 + m : 0);
 #pragma unroll
             for (int n = 0; n < COUT; ++n) {
@@ -594,8 +594,11 @@ __global__ void __launch_bounds__(CT, 1) k_conv3d(const __grid_constant__ CUtens
 // its partial sums to a workspace row and a second kernel adds the rows to dW
 // in CTA order, so the result does not depend on timing.
 //
-// Bound by L2 reads (42 KB a segment for 32 input channels) and the hand-offs
-// of three stages; 128x128x64, us: 16->32 117, 32->32 143, 32->16 129.  The
+// No unit is full: 32->32 at 128x128x64, a segment takes 2050 cycles of its SM,
+// 720 of them with the tensor pipe active (48 an MMA of N = 96); L2 is at 37 %
+// (42 KB a segment), DRAM at 12 %, issue at 12 %.  What is left is the chain of a
+// segment, boxes and halo copies, hand-off, 15 MMAs, hand-off, of which three
+// are in flight.  128x128x64, us: 16->32 117, 32->32 143, 32->16 129.  The
 // form that transposed both operands through registers took 463, 657 and 605,
 // this one with every voxel by cp.async 151, 241 and 231.  Marching along y with
 // 128-voxel segments and the roles of the operands exchanged took 137, 146 and

@@ -16,7 +16,7 @@
 #pragma once
 
 #ifndef MHD3D_MINB
-#define MHD3D_MINB 3   // FP64 stage CTAs per SM: 3 x 128 threads x 168 registers, 3 x 72 KB shared
+#define MHD3D_MINB 3   // FP64 stage CTAs per SM: 3 x 128 threads x up to 168 registers, 3 x 74 to 77 KB shared (8 fields)
 #endif
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -10,8 +10,9 @@
 // Work decomposition of both: a CTA owns a TX x TY tile of (x,y) columns and
 // a chunk of z planes and marches down the chunk.  The raw fields of each
 // plane arrive by TMA (cp.async.bulk.tensor, one 4-D box per plane: x with
-// the periodic halo, y with the halo, one plane, all fields) into a four-slot
-// ring; 1/RO of the planes in use sits in a ring next to it.  Velocities and
+// the periodic halo, y with the halo, one plane, all fields) into a ring of four
+// slots (five in the march's stages without Z); 1/RO of the planes in use sits
+// in a ring next to it.  Velocities and
 // pressure are formed where they are used, from the same two operands
 // FLUXES multiplies (3dmhdsub.f:1386-1425).  The Z tile of the plane (stages
 // 2, 3) arrives by its own TMA box a plane ahead.  The wall planes take BCON

@@ -12,15 +12,17 @@
 //
 // GEN instances (StageArgs.general) are for what the others leave out to stay
 // as fast as they are: Z stored by stage 1, and wall values that BCON does not
-// rewrite (BZ with IBC not 0, TT on the top wall with ITC=3).
+// rewrite (BZ with IBC not 0, TT on the top wall with ITC=3).  A step by them
+// takes 10.08 ms at 512x512x256 against 9.43, 1256 us at 256x256x128 against 1207.
 //
 // Bound by DRAM traffic in flight (12 warps an SM, two planes in the ring
 // beyond the two in use, three in stage 1) together with the latency of a
-// plane's 705-830 instructions.  Measured at 512x512x256 (ms a step; stages):
-// one plane in flight, planes k-1, k, k+1 read for every cell 10.61 (3.18 /
-// 3.58 / 3.79); the march 9.76 (2.98 / 3.31 / 3.37); stage 1 without Z, rows
-// on 128-byte lines and 32-plane chunks 9.39 (2.62 / 3.24 / 3.39).  At
-// 256x256x128 1581, 1413 and 1241 us.
+// plane's instructions (690, 808 and 870 in stages 1, 2, 3 with a magnetic
+// field).  Measured at 512x512x256 (ms a step; stages): one plane in flight,
+// planes k-1, k, k+1 read for every cell 10.61 (3.18 / 3.58 / 3.79); the march
+// 9.76 (2.98 / 3.31 / 3.37); stage 1 without Z, rows on 128-byte lines and
+// 32-plane chunks 9.39 (2.62 / 3.24 / 3.39).  At 256x256x128 1581, 1413 and
+// 1241 us; 1207 with the chunks that z_chunks now chooses there.
 // Tried against the march in one run: 4 CTAs an SM at 128 registers with a
 // three-slot ring and one Z slot 1425 us and 10.4 ms; 32x8 tiles, 2 CTAs an
 // SM, three slots 1410 us and 10.16 ms, four slots and one Z slot 1529 us and
